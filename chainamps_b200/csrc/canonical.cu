@@ -438,6 +438,10 @@ int build_canonical(Heff& H) {
   C->sW1 = std::move(P.sW1);
   C->sW2 = std::move(P.sW2);
   C->sR = std::move(P.sR);
+  // real MPO blocks (operators with real matrix elements): the W stages then
+  // need two real products per complex one
+  C->sW1.a_real = C->sW2.a_real =
+      std::all_of(P.ops_im.begin(), P.ops_im.end(), [](double v) { return v == 0.0; });
   for (GemmPlan* p : {&C->sL, &C->sW1, &C->sW2, &C->sR})
     if ((rc = p->upload(st)) != CMPS_OK) return bail(rc);
   C->flops = P.flops;
@@ -449,6 +453,7 @@ int build_canonical32(Heff& H) {
   if (!C) return fail(CMPS_ERR_STATE, "canonical-order plans not built");
   if (C->have32) return CMPS_OK;
   cudaStream_t st = H.ctx->stream;
+  for (GemmPlan* p : {&C->sL, &C->sW1, &C->sW2, &C->sR}) CMPS_TRY(p->tile_fp32(st));
   CMPS_TRY(C->ops32.alloc(C->ops.len));
   CMPS_TRY(C->L32.alloc(H.L.data.len));
   CMPS_TRY(C->R32.alloc(H.R.data.len));
@@ -512,15 +517,15 @@ int autotune_canonical(Heff& H, bool fp32, cudaStream_t st, TuneStats* stats) {
   if (fp32) {
     if (!C->have32) rc = fail(CMPS_ERR_STATE, "canonical-order FP32 operands not prepared");
     if (rc == CMPS_OK) rc = to_fp32(in.re(), in.im(), H.in_len, C->x32, st);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sL, 20, [&] { return launch_cgemm_fp32(C->sL, C->L32, C->x32, C->xz32, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sW1, 21, [&] { return launch_cgemm_fp32(C->sW1, C->ops32, C->xz32, C->y32, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sW2, 22, [&] { return launch_cgemm_fp32(C->sW2, C->ops32, C->y32, C->xz32, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sR, 23, [&] { return launch_cgemm_fp32(C->sR, C->xz32, C->R32, C->o32, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sL, 20, true, [&] { return launch_cgemm_fp32(C->sL, C->L32, C->x32, C->xz32, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sW1, 21, true, [&] { return launch_cgemm_fp32(C->sW1, C->ops32, C->xz32, C->y32, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sW2, 22, true, [&] { return launch_cgemm_fp32(C->sW2, C->ops32, C->y32, C->xz32, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sR, 23, true, [&] { return launch_cgemm_fp32(C->sR, C->xz32, C->R32, C->o32, st); }, st, stats);
   } else {
-    rc = autotune_plan(C->sL, 10, [&] { return launch_zgemm_fp64(C->sL, false, false, H.L.data, in, C->xz, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sW1, 11, [&] { return launch_zgemm_fp64(C->sW1, false, false, C->ops, C->xz, C->y, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sW2, 12, [&] { return launch_zgemm_fp64(C->sW2, false, false, C->ops, C->y, C->xz, st); }, st, stats);
-    if (rc == CMPS_OK) rc = autotune_plan(C->sR, 13, [&] { return launch_zgemm_fp64(C->sR, false, false, C->xz, H.R.data, out, st); }, st, stats);
+    rc = autotune_plan(C->sL, 10, false, [&] { return launch_zgemm_fp64(C->sL, false, false, H.L.data, in, C->xz, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sW1, 11, false, [&] { return launch_zgemm_fp64(C->sW1, false, false, C->ops, C->xz, C->y, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sW2, 12, false, [&] { return launch_zgemm_fp64(C->sW2, false, false, C->ops, C->y, C->xz, st); }, st, stats);
+    if (rc == CMPS_OK) rc = autotune_plan(C->sR, 13, false, [&] { return launch_zgemm_fp64(C->sR, false, false, C->xz, H.R.data, out, st); }, st, stats);
   }
   in.d = out.d = nullptr;
   return rc;

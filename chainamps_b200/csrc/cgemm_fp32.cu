@@ -7,8 +7,9 @@
 // precision buys here.
 //
 // Same work description as zgemm_grouped_fp64 (GemmTask / GemmTerm /
-// GemmTile, K-concatenated terms, the two-level N index) and the same tile
-// shapes (64 x 64, 32 x 128, 128 x 32), so one plan drives both precisions.
+// GemmTile, K-concatenated terms, the two-level N index), so one plan drives
+// both precisions, with whole tiles of 64 x 64, 32 x 128 or 128 x 32 of its
+// own (GemmPlan::tile_fp32).
 // 128 threads; thread (tm, tn) owns the 8 x 4 complex outputs (tm + i TM,
 // tn + j TN): shared-memory reads and output stores run along consecutive
 // threads.  Operands are staged global -> shared with 4-byte cp.async
@@ -189,11 +190,11 @@ template <int BM, int BN, bool NSPLIT>
 int launch32(const GemmPlan& p, const Planar32& A, const Planar32& B, Planar32& C, cudaStream_t st) {
   using T = Tile32<BM, BN>;
   CMPS_TRY(ensure_smem_optin((const void*)cgemm_grouped_fp32<BM, BN, NSPLIT>, (int)T::SMEM_BYTES));
-  if (p.tiles.empty()) return CMPS_OK;
-  const int64_t ntiles = (int64_t)p.tiles.size();
+  if (p.t32.n == 0) return CMPS_OK;
+  const int64_t ntiles = p.t32.n;
   if (ntiles > 0x7fffffff) return fail(CMPS_ERR_ARG, "too many GEMM tiles");
   cgemm_grouped_fp32<BM, BN, NSPLIT><<<(unsigned)ntiles, NT, T::SMEM_BYTES, st>>>(
-      p.d_tiles, p.d_tasks, p.d_terms, A.re(), A.im(), B.re(), B.im(), C.re(), C.im());
+      p.t32.d, p.d_tasks, p.d_terms, A.re(), A.im(), B.re(), B.im(), C.re(), C.im());
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }
@@ -242,11 +243,11 @@ void Planar32::release() {
 }
 
 int launch_cgemm_fp32(const GemmPlan& p, const Planar32& A, const Planar32& B, Planar32& C, cudaStream_t st) {
-  switch (p.shape) {
+  switch (p.t32.shape) {
     case 0: return launch32_shape<64, 64>(p, A, B, C, st);
     case 1: return launch32_shape<32, 128>(p, A, B, C, st);
     case 2: return launch32_shape<128, 32>(p, A, B, C, st);
-    default: return fail(CMPS_ERR_STATE, "GEMM plan not uploaded (no tile shape)");
+    default: return fail(CMPS_ERR_STATE, "GEMM plan without FP32 tiles");
   }
 }
 

@@ -970,9 +970,9 @@ int Heff::autotune(TuneStats* stats) {
   in.len = in_len;
   out.d = y.d;
   out.len = out_len;
-  int rc = autotune_plan(stage1, 1, [&] { return launch_zgemm_fp64(stage1, false, false, LP, in, T, st); }, st, stats);
+  int rc = autotune_plan(stage1, 1, false, [&] { return launch_zgemm_fp64(stage1, false, false, LP, in, T, st); }, st, stats);
   if (rc == CMPS_OK)
-    rc = autotune_plan(stage2, 2, [&] { return launch_zgemm_fp64(stage2, false, false, T, RP, out, st); }, st, stats);
+    rc = autotune_plan(stage2, 2, false, [&] { return launch_zgemm_fp64(stage2, false, false, T, RP, out, st); }, st, stats);
   in.d = out.d = nullptr;
   return rc;
 }

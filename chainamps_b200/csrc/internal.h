@@ -154,25 +154,35 @@ struct GemmTerm {
   int64_t a_off, b_off;
   int32_t k, lda, ldb, ldb_out;
 };
+// One CTA's part of a task.  cut (FP64 launch): rows and columns in slices
+// of 8 and the warps' share of them, sm | sn << 6 | log2(warps along M) << 12
+// | slices per warp along M << 14 | along N << 20.
 struct GemmTile {
-  int32_t task, m0, n0, pad;
+  int32_t task, m0, n0, cut;
+};
+struct GemmTiles {
+  GemmTile* d = nullptr;
+  int64_t n = 0;
+  int shape = -1;
 };
 
 struct GemmPlan {
   std::vector<GemmTask> tasks;
   std::vector<GemmTerm> terms;
-  std::vector<GemmTile> tiles;
   GemmTask* d_tasks = nullptr;
   GemmTerm* d_terms = nullptr;
-  GemmTile* d_tiles = nullptr;
   double flops = 0.0;
   bool nsplit = false;  // tasks use the two-level N index (n_in > 0)
-  int shape = -1;       // output tile shape (gemm_shape_m / _n), chosen by upload
-  // Picks the tile shape for these tasks, splits them into tiles and copies
-  // the plan to the device.
+  bool a_real = false;  // the A operand's imaginary plane is zero
+  // The tiles of the FP64 launch (zgemm_fp64.cu), made by upload, and of the
+  // FP32 one (cgemm_fp32.cu), made by tile_fp32 where a plan runs in FP32.
+  GemmTiles t64, t32;
+  // Copies the plan to the device and cuts its tasks into tiles of the shape
+  // that its sizes ask for.
   int upload(cudaStream_t st);
+  int tile_fp32(cudaStream_t st);
   // The tiles again for another shape (an uploaded plan; tasks and terms unchanged).
-  int retile(int shape, cudaStream_t st);
+  int retile(bool fp32, int shape, cudaStream_t st);
   // Host check, before any launch, that every operand and output range lies
   // inside its buffer (lengths in complex elements).
   int validate(bool a_h, bool b_h, int64_t a_len, int64_t b_len, int64_t c_len, const char* what) const;
@@ -188,7 +198,8 @@ struct TuneStats {
   int tuned = 0, cached = 0;
   double ms_heuristic = 0.0, ms_best = 0.0;  // per launch, summed over the tuned plans
 };
-int autotune_plan(GemmPlan& p, int role, const std::function<int()>& run, cudaStream_t st, TuneStats* stats);
+int autotune_plan(GemmPlan& p, int role, bool fp32, const std::function<int()>& run, cudaStream_t st,
+                  TuneStats* stats);
 
 // Block AXPY lists: dst block = sum_t w_t * src_t (same shapes).
 struct AxpyBlock {
@@ -201,9 +212,6 @@ struct AxpyTerm {
 };
 
 // ---- kernels (launchers) ---------------------------------------------------
-// output tile shapes of zgemm_grouped_fp64 (GemmPlan::shape)
-int gemm_shape_m(int shape);
-int gemm_shape_n(int shape);
 int launch_zgemm_fp64(const GemmPlan& p, bool a_h, bool b_h, const Planar& A, const Planar& B,
                       Planar& C, cudaStream_t st);
 // FP32 grouped complex GEMM (cgemm_fp32.cu): the same plans as

@@ -6,13 +6,43 @@
 // term has its own A block, B block and K -- the K-concatenation that turns
 // the charge-sector structure of H_eff (sum over MPO indices and physical
 // states) into a single accumulation.  Complex operands are stored as two
-// planes (re, im) of one allocation; a complex MAC is four real DMMAs.
-// Operands are staged global -> shared with 8-byte cp.async (zero-filled
-// outside the block), double buffered.  op(A) is A or A^H (A stored K x M),
+// planes (re, im) of one allocation.  op(A) is A or A^H (A stored K x M),
 // op(B) is B or B^H (B stored N x K), all row-major with leading dimensions.
 // NSPLIT: the N index of B and C is two-level (GemmTask::n_in), so one task
 // can run over several equally strided column ranges, e.g. the rows of
 // every state of one charge class, or one column class of every row.
+//
+// The FP64 pipe (36.6 TFLOP/s measured for DMMA alone) is the bound of every
+// plan whose blocks are not tiny: a DMMA holds its sub-core's pipe for 16
+// cycles, so what counts is how many DMMAs are issued, and that there is
+// always a warp ready to issue one.
+//  * Trimmed tiles.  Charge sectors have any size (2, 9, 27, 61, 99, 117 on
+//    the ladder at chi = 512), so whole 64 x 64 tiles did 1.40 x the useful
+//    work there, 2.5 x on 40 uneven sectors and 4.5 x on the XXZ chain.  A
+//    tile therefore carries its own number of 8-row and 8-column slices, a
+//    task is cut into tiles of equal slice counts, K is run in steps of 4,
+//    and the slices of a tile are dealt out evenly over its four warps in
+//    the best of the arrangements 4 x 1, 2 x 2, 1 x 4 (GemmTile::cut).  The
+//    work then is 1.07 x, 1.13 x and 1.09 x the useful one.
+//  * Three multiplications per complex product.  With P1 = Ar Br, P2 = Ai Bi
+//    and P3 = (Ar + Ai)(Br + Bi), Re = P1 - P2 and Im = P3 - P1 - P2: 3 DMMAs
+//    per slice pair and k-step instead of 4 (the sums are one DADD per
+//    fragment).  P1, P2 and P3 are folded into the result every kFold values
+//    of K, so that rounding errors do not grow along all of K: against exact
+//    sums the error is 1.01 x that of the four-product chain at K = 128 and
+//    0.25 x at K = 2400; whole matvecs are 0.3 to 0.8 x as far off.
+//  * AREAL: a plan whose A operand has no imaginary part (the MPO blocks of
+//    real operators) needs two products, Ar Br and Ar Bi, and no folding.
+//  * Four CTAs of four warps per SM, each with a ring of three 16 KB stages
+//    filled by 8-byte cp.async (block offsets and leading dimensions have any
+//    parity) and one barrier per 16 values of K.
+// Before (64 x 64 tiles, four products, two CTAs per SM) and now, per matvec:
+// ladder at chi = 512 11.8 and 9.4 ms, Ising chains at chi = 64 10.8 and 5.7
+// ms, 40 uneven sectors 3.4 and 1.5 ms.  The DMMA pipe is 49 to 63% busy; the
+// rest goes to fragment and operand loads that the warps issue between DMMAs.
+//
+// An element's value does not depend on the tile shape or on how tasks are
+// cut: the order of its DMMAs and folds is fixed by its terms alone.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -32,32 +62,34 @@ namespace cmps {
 
 namespace {
 
-// Output tile BM x BN, four warps of 32 x 32 each (WN = BN / 32 across N).
-// Shapes: 64 x 64 (square blocks), 32 x 128 (tasks with M <= 32: a charge
-// class of 32 states, a small a0 sector) and 128 x 32 (tasks with N <= 32).
-// Shared-memory rows are padded to BM + 4 / BN + 4 doubles (= 4 mod 16):
-// conflict-free 8-byte fragment reads.
+// Output tile of up to BM x BN, a warp holds at most WI x WJ slices of 8 x 8.
+// An operand is staged as it is stored, unpadded: rows of 16 values of K, or
+// rows of BM / BN elements per value of K.  The position inside a row is
+// XORed with 4 * (row mod 4), which makes the 8-byte fragment reads free of
+// bank conflicts and keeps four 48 KB rings on an SM.
 constexpr int BK = 16;
 constexpr int NTHREADS = 128;
-constexpr int STAGES = 2;
-template <int BM, int BN>
+constexpr int STAGES = 3;
+constexpr int kFold = 128;  // values of K between two folds of the three products
+template <int BM_, int BN_, int WI_, int WJ_, int CTAS_>
 struct Tile {
-  static_assert(BM % 32 == 0 && BN % 32 == 0 && (BM / 32) * (BN / 32) == 4, "four 32 x 32 warp tiles");
-  static constexpr int WN = BN / 32;
-  static constexpr int LDA = BM + 4, LDB = BN + 4;
-  static constexpr int PLANE_A = BK * LDA, PLANE_B = BK * LDB;  // doubles per plane per stage
+  static constexpr int BM = BM_, BN = BN_, WI = WI_, WJ = WJ_, CTAS = CTAS_;
+  static constexpr int PLANE_A = BM * BK, PLANE_B = BN * BK;  // doubles per plane per stage
   static constexpr int STAGE_DOUBLES = 2 * PLANE_A + 2 * PLANE_B;  // A re, A im, B re, B im
   static constexpr size_t SMEM_BYTES = (size_t)STAGES * STAGE_DOUBLES * sizeof(double);
 };
+using TileQ = Tile<32, 32, 2, 2, 4>;
+using TileS = Tile<32, 16, 2, 1, 4>;  // plans with too few tiles to fill the GPU
 
-__device__ __forceinline__ void cp_async8(double* smem, const double* gmem, bool pred) {
-  unsigned s = (unsigned)__cvta_generic_to_shared(smem);
+__device__ __forceinline__ void cp_async8(unsigned s, const double* gmem) {
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(s), "l"(gmem));
+}
+__device__ __forceinline__ void cp_async8z(unsigned s, const double* gmem, bool pred) {
   int sz = pred ? 8 : 0;
   asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(s), "l"(gmem), "r"(sz));
 }
 __device__ __forceinline__ void cp_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 __device__ __forceinline__ void cp_wait1() { asm volatile("cp.async.wait_group 1;\n" ::); }
-__device__ __forceinline__ void cp_wait0() { asm volatile("cp.async.wait_group 0;\n" ::); }
 
 __device__ __forceinline__ void dmma(double& d0, double& d1, double a, double b) {
   asm volatile("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0,%1}, {%2}, {%3}, {%0,%1};\n"
@@ -73,209 +105,390 @@ __device__ __forceinline__ int64_t ncol(int n, int n_in, int ld_out) {
   return (int64_t)q * ld_out + (n - q * n_in);
 }
 
-// Issue the cp.async copies of one (term, k-tile) into stage buffer `buf`.
-template <int BM, int BN, bool AH, bool BH, bool NSPLIT>
-__device__ __forceinline__ void load_stage(double* buf, const GemmTerm& t, int k0, int m0, int n0, int M,
-                                           int N, int n_in, const double* __restrict__ Ar,
-                                           const double* __restrict__ Ai, const double* __restrict__ Br,
-                                           const double* __restrict__ Bi) {
-  using T = Tile<BM, BN>;
-  double* sAr = buf;
-  double* sAi = buf + T::PLANE_A;
-  double* sBr = buf + 2 * T::PLANE_A;
-  double* sBi = sBr + T::PLANE_B;
-  const int tid = threadIdx.x;
-  const int K = t.k;
-#pragma unroll
-  for (int j = 0; j < (BM * BK) / NTHREADS; ++j) {
-    int idx = tid + j * NTHREADS;
-    int kk, mm;
-    if (!AH) { kk = idx % BK; mm = idx / BK; }   // A[m][k]: consecutive threads along k
-    else     { kk = idx / BM; mm = idx % BM; }   // A stored [k][m]: along m
-    int gm = m0 + mm, gk = k0 + kk;
-    bool ok = (gm < M) && (gk < K);
-    int64_t o = ok ? (AH ? t.a_off + (int64_t)gk * t.lda + gm : t.a_off + (int64_t)gm * t.lda + gk) : 0;
-    cp_async8(sAr + kk * T::LDA + mm, Ar + o, ok);
-    cp_async8(sAi + kk * T::LDA + mm, Ai + o, ok);
+// One thread's part of an operand's loads into a stage buffer, one element
+// of each plane per pass.  KLANE: the lanes of a 16-thread group run along K
+// and the passes along the other index, 8 apart (A as stored, B^H); else the
+// lanes run along the other index (EXT of them) and the passes along K.
+// Elements of rows or columns outside the block are not loaded: they only
+// reach outputs that are not stored.  K past the term's end, up to the next
+// multiple of 4, is filled with zeros.
+template <int EXT, bool KLANE, bool REAL>
+struct Loader {
+  static constexpr int PASSES = KLANE ? EXT / 8 : BK * EXT / NTHREADS;
+  static constexpr int APART = KLANE ? 8 : NTHREADS / EXT;
+  static constexpr unsigned PLANE = EXT * BK * sizeof(double);
+  static constexpr unsigned SSTEP = APART * (KLANE ? BK : EXT) * sizeof(double);
+  const double *re, *im;
+  int ld;       // leading dimension of the current term
+  int n;        // passes that this thread loads: all whose element exists
+  unsigned s;   // where pass 0 lands in the stage buffer
+  static __device__ __forceinline__ int lane() { return threadIdx.x % (KLANE ? BK : EXT); }
+  static __device__ __forceinline__ int row() { return threadIdx.x / (KLANE ? BK : EXT); }
+  // slices: of this tile along the operand's other index; left: elements there
+  __device__ __forceinline__ void open_tile(unsigned ring, int slices, int left) {
+    const int l = lane(), r = row();
+    n = KLANE ? min(slices, (left - r + 7) >> 3) : (l < left && l < 8 * slices ? PASSES : 0);
+    s = ring + (r * (KLANE ? BK : EXT) + (l ^ (r & 3) << 2)) * (unsigned)sizeof(double);
   }
+  // origin: element (0, 0) of this tile in the term's block; at: this
+  // thread's offset from it along the other index when the lanes run there
+  __device__ __forceinline__ void open_term(const double* origin, int64_t plane, int ld_, int64_t at) {
+    ld = ld_;
+    re = origin + (int64_t)row() * ld + (KLANE ? lane() : at);
+    if (!REAL) im = re + plane;
+  }
+  __device__ __forceinline__ void load(unsigned stage, int kl) {
+    const unsigned d = s + stage;
+    if (kl == BK) {
 #pragma unroll
-  for (int j = 0; j < (BN * BK) / NTHREADS; ++j) {
-    int idx = tid + j * NTHREADS;
-    int kk, nn;
-    if (!BH) { kk = idx / BN; nn = idx % BN; }   // B[k][n]: along n
-    else     { kk = idx % BK; nn = idx / BK; }   // B stored [n][k]: along k
-    int gn = n0 + nn, gk = k0 + kk;
-    bool ok = (gn < N) && (gk < K);
-    int64_t o = ok ? (BH ? t.b_off + (int64_t)gn * t.ldb + gk
-                         : t.b_off + (int64_t)gk * t.ldb + ncol<NSPLIT>(gn, n_in, t.ldb_out))
-                   : 0;
-    cp_async8(sBr + kk * T::LDB + nn, Br + o, ok);
-    cp_async8(sBi + kk * T::LDB + nn, Bi + o, ok);
+      for (int j = 0; j < PASSES; ++j)
+        if (j < n) {
+          cp_async8(d + j * SSTEP, re + (int64_t)ld * (APART * j));
+          if (!REAL) cp_async8(d + j * SSTEP + PLANE, im + (int64_t)ld * (APART * j));
+        }
+    } else {
+      const int kl4 = (kl + 3) & ~3;
+#pragma unroll
+      for (int j = 0; j < PASSES; ++j) {
+        const int k = KLANE ? lane() : row() + APART * j;
+        if (j < n && k < kl4) {
+          const int64_t o = k < kl ? (int64_t)ld * (APART * j) : 0;
+          cp_async8z(d + j * SSTEP, re + o, k < kl);
+          if (!REAL) cp_async8z(d + j * SSTEP + PLANE, im + o, k < kl);
+        }
+      }
+    }
+    re += KLANE ? (int64_t)BK : (int64_t)ld * BK;
+    if (!REAL) im += KLANE ? (int64_t)BK : (int64_t)ld * BK;
+  }
+};
+
+// The arrangement of the four warps over a tile of sm x sn slices, 2^wml of
+// them along M, with the fewest slice pairs hm x hn on the busiest warp.
+template <class T>
+__host__ __device__ __forceinline__ void arrange(int sm, int sn, int& hm, int& hn, int& wml) {
+  int best = 1 << 20;
+  hm = hn = wml = 0;
+#pragma unroll
+  for (int x = 0; x <= 2; ++x) {
+    const int a = (sm + (1 << x) - 1) >> x, b = (sn + (4 >> x) - 1) >> (2 - x);
+    if (a <= T::WI && b <= T::WJ && a * b < best) {
+      best = a * b;
+      hm = a;
+      hn = b;
+      wml = x;
+    }
   }
 }
 
-template <int BM, int BN, bool AH, bool BH, bool NSPLIT>
-__global__ void __launch_bounds__(NTHREADS, 2)
+// A warp's accumulators: the result and, unless AREAL, the three products
+// since the last fold.
+template <class T>
+struct Acc {
+  double cr[T::WI][T::WJ][2], ci[T::WI][T::WJ][2];
+  double p1[T::WI][T::WJ][2], p2[T::WI][T::WJ][2], p3[T::WI][T::WJ][2];
+};
+
+// One stage of kl values of K for a warp's NI x NJ slices, straight-line.
+template <class T, bool AH, bool BH, bool AREAL, int NI, int NJ>
+__device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, int j0, int kl) {
+  const int lane = threadIdx.x & 31;
+  const int gid = lane >> 2, tig = lane & 3;
+  const double* sA = buf + (AH ? tig * T::BM : (i0 * 8 + gid) * BK + tig);
+  const double* sB = buf + 2 * T::PLANE_A + (BH ? (j0 * 8 + gid) * BK + tig : tig * T::BN);
+  const int xk = (gid & 3) << 2, xt = tig << 2;  // the rows' XOR patterns
+#pragma unroll
+  for (int kk = 0; kk < BK; kk += 4) {
+    if (kk >= kl) break;
+    double ar[NI], ai[NI], as[NI], br[NJ], bi[NJ];
+#pragma unroll
+    for (int i = 0; i < NI; ++i) {
+      const int o = AH ? kk * T::BM + (((i0 + i) * 8 + gid) ^ xt) : 8 * i * BK + (kk ^ xk);
+      ar[i] = sA[o];
+      if (!AREAL) {
+        ai[i] = AH ? -sA[o + T::PLANE_A] : sA[o + T::PLANE_A];
+        as[i] = ar[i] + ai[i];
+      }
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j) {
+      const int o = BH ? 8 * j * BK + (kk ^ xk) : kk * T::BN + (((j0 + j) * 8 + gid) ^ xt);
+      br[j] = sB[o];
+      bi[j] = BH ? -sB[o + T::PLANE_B] : sB[o + T::PLANE_B];
+    }
+#pragma unroll
+    for (int j = 0; j < NJ; ++j)
+#pragma unroll
+      for (int i = 0; i < NI; ++i) {
+        if (AREAL) {
+          dmma(c.cr[i][j][0], c.cr[i][j][1], ar[i], br[j]);
+          dmma(c.ci[i][j][0], c.ci[i][j][1], ar[i], bi[j]);
+        } else {
+          dmma(c.p1[i][j][0], c.p1[i][j][1], ar[i], br[j]);
+          dmma(c.p2[i][j][0], c.p2[i][j][1], ai[i], bi[j]);
+          dmma(c.p3[i][j][0], c.p3[i][j][1], as[i], br[j] + bi[j]);
+        }
+      }
+  }
+}
+
+template <class T, bool AH, bool BH, bool NSPLIT, bool AREAL>
+__global__ void __launch_bounds__(NTHREADS, T::CTAS)
 zgemm_grouped_fp64(const GemmTile* __restrict__ tiles, const GemmTask* __restrict__ tasks,
-                   const GemmTerm* __restrict__ terms, const double* __restrict__ Ar,
-                   const double* __restrict__ Ai, const double* __restrict__ Br,
-                   const double* __restrict__ Bi, double* __restrict__ Cr, double* __restrict__ Ci) {
+                   const GemmTerm* __restrict__ terms, const double* __restrict__ Ar, int64_t planeA,
+                   const double* __restrict__ Br, int64_t planeB, double* __restrict__ Cr, int64_t planeC) {
   extern __shared__ double smem[];
   const GemmTile tile = tiles[blockIdx.x];
   const GemmTask task = tasks[tile.task];
-  const int m0 = tile.m0, n0 = tile.n0, M = task.m, N = task.n;
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  using T = Tile<BM, BN>;
-  const int wm = warp / T::WN, wn = warp % T::WN;
+  const int lane = threadIdx.x & 31;
   const int gid = lane >> 2, tig = lane & 3;
-
-  double accr[4][4][2], acci[4][4][2];
-#pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      accr[i][j][0] = accr[i][j][1] = 0.0;
-      acci[i][j][0] = acci[i][j][1] = 0.0;
-    }
-
-  // iteration cursor over (term, k-tile)
-  int cur_t = task.t0, cur_k = 0;
-  int nxt_t = cur_t, nxt_k = 0;
-  bool have = cur_t < task.t1;
-  if (have) {
-    GemmTerm t = terms[cur_t];
-    load_stage<BM, BN, AH, BH, NSPLIT>(smem, t, 0, m0, n0, M, N, task.n_in, Ar, Ai, Br, Bi);
-    cp_commit();
-    nxt_k = BK;
-    if (nxt_k >= t.k) { nxt_t = cur_t + 1; nxt_k = 0; }
+  const int m0 = tile.m0, n0 = tile.n0, sm = tile.cut & 63, sn = tile.cut >> 6 & 63;
+  Loader<T::BM, !AH, AREAL> la;
+  Loader<T::BN, BH, false> lb;
+  const unsigned ring = (unsigned)__cvta_generic_to_shared(smem);
+  la.open_tile(ring, sm, task.m - m0);
+  lb.open_tile(ring + 2 * T::PLANE_A * (unsigned)sizeof(double), sn, task.n - n0);
+  int nq = 0, nr = 0;  // two-level index of this thread's B column
+  if (NSPLIT) {
+    const int gn = n0 + (int)threadIdx.x % T::BN;
+    nq = gn / task.n_in;
+    nr = gn - nq * task.n_in;
   }
-  int stage = 0;
-  while (have) {
-    bool more = nxt_t < task.t1;
-    if (more) {
-      GemmTerm t = terms[nxt_t];
-      load_stage<BM, BN, AH, BH, NSPLIT>(smem + (stage ^ 1) * T::STAGE_DOUBLES, t, nxt_k, m0, n0, M, N, task.n_in, Ar,
-                                         Ai, Br, Bi);
-      cp_commit();
-      cp_wait1();
-    } else {
-      cp_wait0();
+  // this warp's share of the tile's slices; the warps' roles rotate with the
+  // block, so that the larger shares of resident CTAs do not meet on one
+  // sub-core
+  const int wml = tile.cut >> 12 & 3, hm = tile.cut >> 14 & 63, hn = tile.cut >> 20;
+  const int role = ((threadIdx.x >> 5) + blockIdx.x) & 3;
+  const int i0 = (role & ((1 << wml) - 1)) * hm, j0 = (role >> wml) * hn;
+  const int ni = min(hm, sm - i0), nj = ni > 0 ? min(hn, sn - j0) : 0;
+
+  Acc<T> c;
+#pragma unroll
+  for (int i = 0; i < T::WI; ++i)
+#pragma unroll
+    for (int j = 0; j < T::WJ; ++j)
+#pragma unroll
+      for (int e = 0; e < 2; ++e)
+        c.cr[i][j][e] = c.ci[i][j][e] = c.p1[i][j][e] = c.p2[i][j][e] = c.p3[i][j][e] = 0.0;
+
+  // issue cursor over (term, k): fills stage buffer b and returns its values of K
+  int it = task.t0, left = 0;
+  auto issue = [&](int b) -> int {
+    if (left <= 0 && it < task.t1) {
+      const GemmTerm t = terms[it++];
+      left = t.k;
+      la.open_term(Ar + t.a_off + (AH ? (int64_t)m0 : (int64_t)m0 * t.lda), planeA, t.lda, la.lane());
+      lb.open_term(Br + t.b_off + (NSPLIT ? 0 : BH ? (int64_t)n0 * t.ldb : (int64_t)n0), planeB, t.ldb,
+                   NSPLIT ? (int64_t)nq * t.ldb_out + nr : (int64_t)lb.lane());
     }
-    __syncthreads();
-    const double* sAr = smem + stage * T::STAGE_DOUBLES;
-    const double* sAi = sAr + T::PLANE_A;
-    const double* sBr = sAr + 2 * T::PLANE_A;
-    const double* sBi = sBr + T::PLANE_B;
-#pragma unroll
-    for (int kk = 0; kk < BK; kk += 4) {
-      double ar[4], ai[4], nai[4], br[4], bi[4];
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        int mm = wm * 32 + i * 8 + gid;
-        ar[i] = sAr[(kk + tig) * T::LDA + mm];
-        ai[i] = sAi[(kk + tig) * T::LDA + mm];
-        if (AH) ai[i] = -ai[i];
-        nai[i] = -ai[i];
+    const int kl = max(0, min(BK, left));
+    if (kl) {
+      const unsigned stage = (unsigned)(b * T::STAGE_DOUBLES * sizeof(double));
+      la.load(stage, kl);
+      lb.load(stage, kl);
+      left -= BK;
+    }
+    cp_commit();
+    return kl;
+  };
+  int len0 = issue(0), len1 = issue(1);
+  int buf = 0, since = 0;
+  while (len0 > 0) {
+    cp_wait1();
+    __syncthreads();  // stage `buf` has landed for every thread, and the stage refilled below has been read by all
+    const int len2 = issue(buf == 0 ? 2 : buf - 1);
+    const double* sbuf = smem + buf * T::STAGE_DOUBLES;
+    // at most WI x WJ slices, one straight-line body each
+    if (nj == 2) {
+      if constexpr (T::WJ >= 2) {
+        if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 2>(c, sbuf, i0, j0, len0);
+        else mma_stage<T, AH, BH, AREAL, 1, 2>(c, sbuf, i0, j0, len0);
       }
-#pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        int nn = wn * 32 + j * 8 + gid;
-        br[j] = sBr[(kk + tig) * T::LDB + nn];
-        bi[j] = sBi[(kk + tig) * T::LDB + nn];
-        if (BH) bi[j] = -bi[j];
-      }
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) {
-          dmma(accr[i][j][0], accr[i][j][1], ar[i], br[j]);
-          dmma(accr[i][j][0], accr[i][j][1], nai[i], bi[j]);
-          dmma(acci[i][j][0], acci[i][j][1], ar[i], bi[j]);
-          dmma(acci[i][j][0], acci[i][j][1], ai[i], br[j]);
-        }
+    } else if (nj == 1) {
+      if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 1>(c, sbuf, i0, j0, len0);
+      else mma_stage<T, AH, BH, AREAL, 1, 1>(c, sbuf, i0, j0, len0);
     }
-    __syncthreads();
-    // advance
-    have = more;
-    if (more) {
-      cur_t = nxt_t;
-      cur_k = nxt_k;
-      GemmTerm t = terms[cur_t];
-      nxt_k = cur_k + BK;
-      nxt_t = cur_t;
-      if (nxt_k >= t.k) { nxt_t = cur_t + 1; nxt_k = 0; }
-      stage ^= 1;
+    since += len0;
+    if (!AREAL && (since >= kFold || len1 == 0)) {
+      since = 0;
+#pragma unroll
+      for (int i = 0; i < T::WI; ++i)
+#pragma unroll
+        for (int j = 0; j < T::WJ; ++j)
+#pragma unroll
+          for (int e = 0; e < 2; ++e) {
+            c.cr[i][j][e] += c.p1[i][j][e] - c.p2[i][j][e];
+            c.ci[i][j][e] += (c.p3[i][j][e] - c.p1[i][j][e]) - c.p2[i][j][e];
+            c.p1[i][j][e] = c.p2[i][j][e] = c.p3[i][j][e] = 0.0;
+          }
     }
+    len0 = len1;
+    len1 = len2;
+    buf = buf == STAGES - 1 ? 0 : buf + 1;
   }
   // epilogue
+  const int gm0 = m0 + i0 * 8 + gid, gn0 = n0 + j0 * 8 + 2 * tig;
+  const int rows = task.m - gm0, cols = task.n - gn0;
+  double* row = Cr + task.c_off + (int64_t)gm0 * task.ldc;
+  int64_t col[T::WJ][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int j = 0; j < T::WJ; ++j)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
+    for (int e = 0; e < 2; ++e) col[j][e] = ncol<NSPLIT>(gn0 + 8 * j + e, task.n_in, task.ldc_out);
 #pragma unroll
-      for (int e = 0; e < 2; ++e) {
-        int gm = m0 + wm * 32 + i * 8 + gid;
-        int gn = n0 + wn * 32 + j * 8 + 2 * tig + e;
-        if (gm < M && gn < N) {
-          int64_t o = task.c_off + (int64_t)gm * task.ldc + ncol<NSPLIT>(gn, task.n_in, task.ldc_out);
-          Cr[o] = accr[i][j][e];
-          Ci[o] = acci[i][j][e];
-        }
-      }
+  for (int i = 0; i < T::WI; ++i) {
+    if (i < ni && 8 * i < rows) {
+#pragma unroll
+      for (int j = 0; j < T::WJ; ++j)
+#pragma unroll
+        for (int e = 0; e < 2; ++e)
+          if (j < nj && 8 * j + e < cols) {
+            row[col[j][e]] = c.cr[i][j][e];
+            row[col[j][e] + planeC] = c.ci[i][j][e];
+          }
+    }
+    row += (int64_t)8 * task.ldc;
+  }
 }
 
-template <int BM, int BN, bool AH, bool BH, bool NSPLIT>
+template <class T, bool AH, bool BH, bool NSPLIT, bool AREAL>
 int launch_variant(const GemmPlan& p, const Planar& A, const Planar& B, Planar& C, cudaStream_t st) {
-  using T = Tile<BM, BN>;
-  CMPS_TRY(ensure_smem_optin((const void*)zgemm_grouped_fp64<BM, BN, AH, BH, NSPLIT>, (int)T::SMEM_BYTES));
-  if (p.tiles.empty()) return CMPS_OK;
-  const int64_t ntiles = (int64_t)p.tiles.size();
-  if (ntiles > 0x7fffffff) return fail(CMPS_ERR_ARG, "too many GEMM tiles");
-  zgemm_grouped_fp64<BM, BN, AH, BH, NSPLIT><<<(unsigned)ntiles, NTHREADS, T::SMEM_BYTES, st>>>(
-      p.d_tiles, p.d_tasks, p.d_terms, A.re(), A.im(), B.re(), B.im(), C.re(), C.im());
+  CMPS_TRY(ensure_smem_optin((const void*)zgemm_grouped_fp64<T, AH, BH, NSPLIT, AREAL>, (int)T::SMEM_BYTES));
+  if (p.t64.n <= 0) return CMPS_OK;
+  if (p.t64.n > 0x7fffffff) return fail(CMPS_ERR_ARG, "too many GEMM tiles");
+  zgemm_grouped_fp64<T, AH, BH, NSPLIT, AREAL><<<(unsigned)p.t64.n, NTHREADS, T::SMEM_BYTES, st>>>(
+      p.t64.d, p.d_tasks, p.d_terms, A.re(), A.im() - A.re(), B.re(), B.im() - B.re(), C.re(), C.im() - C.re());
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }
 
-template <int BM, int BN>
+template <class T>
 int launch_shape(const GemmPlan& p, bool a_h, bool b_h, const Planar& A, const Planar& B, Planar& C,
                  cudaStream_t st) {
-  if (p.nsplit) {
-    if (a_h || b_h) return fail(CMPS_ERR_STATE, "two-level N index with a conjugate-transposed operand");
-    return launch_variant<BM, BN, false, false, true>(p, A, B, C, st);
+  if (p.nsplit || p.a_real) {
+    if (a_h || b_h) return fail(CMPS_ERR_STATE, "two-level N index or real A with a conjugate-transposed operand");
+    if (p.nsplit && p.a_real) return launch_variant<T, false, false, true, true>(p, A, B, C, st);
+    if (p.a_real) return launch_variant<T, false, false, false, true>(p, A, B, C, st);
+    return launch_variant<T, false, false, true, false>(p, A, B, C, st);
   }
-  if (!a_h && !b_h) return launch_variant<BM, BN, false, false, false>(p, A, B, C, st);
-  if (a_h && !b_h) return launch_variant<BM, BN, true, false, false>(p, A, B, C, st);
-  if (!a_h && b_h) return launch_variant<BM, BN, false, true, false>(p, A, B, C, st);
-  return launch_variant<BM, BN, true, true, false>(p, A, B, C, st);
+  if (!a_h && !b_h) return launch_variant<T, false, false, false, false>(p, A, B, C, st);
+  if (a_h && !b_h) return launch_variant<T, true, false, false, false>(p, A, B, C, st);
+  if (!a_h && b_h) return launch_variant<T, false, true, false, false>(p, A, B, C, st);
+  return launch_variant<T, true, true, false, false>(p, A, B, C, st);
 }
 
-constexpr int kShapes[3][2] = {{64, 64}, {32, 128}, {128, 32}};
+constexpr int kNumShapes64 = 2;
+constexpr int kShapes32[3][2] = {{64, 64}, {32, 128}, {128, 32}};
+
+// Tiles of at most `most` slices of 8 along an extent of n.
+int parts(int64_t n, int most) { return (int)(((n + 7) / 8 + most - 1) / most); }
 
 }  // namespace
 
-int gemm_shape_m(int shape) { return kShapes[shape][0]; }
-int gemm_shape_n(int shape) { return kShapes[shape][1]; }
-
 int launch_zgemm_fp64(const GemmPlan& p, bool a_h, bool b_h, const Planar& A, const Planar& B, Planar& C,
                       cudaStream_t st) {
-  switch (p.shape) {
-    case 0: return launch_shape<64, 64>(p, a_h, b_h, A, B, C, st);
-    case 1: return launch_shape<32, 128>(p, a_h, b_h, A, B, C, st);
-    case 2: return launch_shape<128, 32>(p, a_h, b_h, A, B, C, st);
+  switch (p.t64.shape) {
+    case 0: return launch_shape<TileQ>(p, a_h, b_h, A, B, C, st);
+    case 1: return launch_shape<TileS>(p, a_h, b_h, A, B, C, st);
     default: return fail(CMPS_ERR_STATE, "GEMM plan not uploaded (no tile shape)");
   }
 }
 
-// Tile shape of a plan, chosen from its own tasks: the shape whose padded
-// work (every task rounded up to whole tiles, times its K) plus a fixed cost
-// per tile (prologue, epilogue, scheduling: the work of 16 k-steps of a
-// 32 x 32 quarter tile) is least.  Ties keep 64 x 64.
-static int pick_shape(const GemmPlan& p) {
+// A tile's cost in SM cycles: its busiest warp's DMMAs (16 cycles each; two
+// or three per slice pair and 4 values of K) or the issue of its loads and
+// fragment reads, whichever is more, plus what its epilogue takes.
+template <class T>
+static double tile_cost(int sm, int sn, double k4, double k16, bool a_real) {
+  int hm, hn, wml;
+  arrange<T>(sm, sn, hm, hn, wml);
+  return std::max(k4 * hm * hn * (a_real ? 32 : 48), 300.0 * k16) + 500.0;
+}
+
+template <class T>
+static double task_cost(const GemmPlan& p, const GemmTask& t, int64_t* ntiles, double* longest) {
+  if (t.m <= 0 || t.n <= 0) return 0.0;
+  double k4 = 0.0, k16 = 0.0;
+  for (int q = t.t0; q < t.t1; ++q) {
+    k4 += (p.terms[q].k + 3) / 4;
+    k16 += (p.terms[q].k + BK - 1) / BK;
+  }
+  const int pm = parts(t.m, T::BM / 8), pn = parts(t.n, T::BN / 8);
+  const int sm = ((t.m + 7) / 8 + pm - 1) / pm, sn = ((t.n + 7) / 8 + pn - 1) / pn;
+  const double c = tile_cost<T>(sm, sn, k4, k16, p.a_real);
+  *ntiles += (int64_t)pm * pn;
+  if (c > *longest) *longest = c;
+  return c;
+}
+
+// Tile shape of a plan in FP64: 32 x 32, or 32 x 16 where the 32 x 32 tiles
+// are too few to fill the GPU evenly -- a launch takes the larger of the
+// tiles' summed cost over 148 SMs and the longest tile beside the others on
+// its SM.  32 x 16 reads each element of A more often, which costs it 8 to
+// 16% on plans of many tiles: ladder at chi = 512, 4.98 + 4.44 ms in 32 x 32
+// and 5.80 + 4.74 ms in 32 x 16; 40 uneven sectors, 0.72 + 0.77 and 0.79 +
+// 0.74 ms; XXZ chain at chi = 250, 24 + 52 and 20 + 34 us.  Larger tiles
+// (64 x 32, 32 x 64) leave room for two CTAs per SM only and lost to 32 x 32
+// on every plan measured, by 2 to 50%.
+template <class T>
+static double launch_cost(const GemmPlan& p) {
+  double sum = 0.0, longest = 0.0;
+  for (const GemmTask& t : p.tasks) {
+    int64_t n = 0;
+    const double c = task_cost<T>(p, t, &n, &longest);
+    sum += c * (double)n;
+  }
+  return std::max(sum / 148.0, longest * T::CTAS);
+}
+static int pick_shape64(const GemmPlan& p) { return launch_cost<TileQ>(p) <= 1.1 * launch_cost<TileS>(p) ? 0 : 1; }
+
+// The tiles of the plan's tasks.  Tasks with long K come first (in octaves of
+// K, so that tasks sharing operands stay neighbours): the launch's last wave
+// is then made of short tiles.
+template <class T>
+static void make_tiles(const GemmPlan& p, std::vector<GemmTile>& out) {
+  std::vector<std::pair<int, int32_t>> order;
+  int64_t total = 0;
+  for (size_t i = 0; i < p.tasks.size(); ++i) {
+    const GemmTask& t = p.tasks[i];
+    if (t.m <= 0 || t.n <= 0) continue;
+    total += (int64_t)parts(t.m, T::BM / 8) * parts(t.n, T::BN / 8);
+    int64_t k = 1;
+    for (int q = t.t0; q < t.t1; ++q) k += (p.terms[q].k + BK - 1) / BK;
+    int oct = 0;
+    while (k >>= 1) ++oct;
+    order.push_back({-oct, (int32_t)i});
+  }
+  std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first < b.first; });
+  out.reserve((size_t)total);
+  for (auto& o : order) {
+    const GemmTask& t = p.tasks[o.second];
+    // slice counts differ by at most one over a task's tiles
+    const int pm = parts(t.m, T::BM / 8), pn = parts(t.n, T::BN / 8);
+    const int64_t sM = (t.m + 7) / 8, sN = (t.n + 7) / 8;
+    for (int a = 0; a < pm; ++a) {
+      const int64_t ma = sM * a / pm;
+      const int sm = (int)(sM * (a + 1) / pm - ma);
+      for (int b = 0; b < pn; ++b) {
+        const int64_t nb = sN * b / pn;
+        const int sn = (int)(sN * (b + 1) / pn - nb);
+        int hm, hn, wml;
+        arrange<T>(sm, sn, hm, hn, wml);
+        out.push_back(GemmTile{o.second, (int32_t)(8 * ma), (int32_t)(8 * nb),
+                               sm | sn << 6 | wml << 12 | hm << 14 | hn << 20});
+      }
+    }
+  }
+}
+
+// Tile shape of a plan in FP32 (cgemm_fp32.cu, whole tiles): the shape whose
+// padded work (every task rounded up to whole tiles, times its K) plus a
+// fixed cost per tile (prologue, epilogue, scheduling: the work of 16 k-steps
+// of a 32 x 32 quarter tile) is least.  Ties keep 64 x 64.
+static int pick_shape32(const GemmPlan& p) {
   double best = 0.0;
   int shape = 0;
   for (int s = 0; s < 3; ++s) {
-    const int bm = kShapes[s][0], bn = kShapes[s][1];
+    const int bm = kShapes32[s][0], bn = kShapes32[s][1];
     double cost = 0.0;
     for (const GemmTask& t : p.tasks) {
       if (t.m <= 0 || t.n <= 0) continue;
@@ -292,15 +505,18 @@ static int pick_shape(const GemmPlan& p) {
   return shape;
 }
 
-int GemmPlan::retile(int s, cudaStream_t st) {
-  if (s < 0 || s > 2) return fail(CMPS_ERR_ARG, "GEMM plan: unknown tile shape");
+int GemmPlan::retile(bool fp32, int s, cudaStream_t st) {
+  if (s < 0 || s >= (fp32 ? 3 : kNumShapes64)) return fail(CMPS_ERR_ARG, "GEMM plan: unknown tile shape");
   if (!d_tasks && !tasks.empty()) return fail(CMPS_ERR_STATE, "GEMM plan not uploaded");
-  const int bm = kShapes[s][0], bn = kShapes[s][1];
   std::vector<GemmTile> nt;
-  for (size_t i = 0; i < tasks.size(); ++i) {
-    const GemmTask& t = tasks[i];
-    for (int m0 = 0; m0 < t.m; m0 += bm)
-      for (int n0 = 0; n0 < t.n; n0 += bn) nt.push_back(GemmTile{(int32_t)i, m0, n0, 0});
+  if (!fp32) {
+    if (s == 0) make_tiles<TileQ>(*this, nt);
+    else make_tiles<TileS>(*this, nt);
+  } else {
+    const int bm = kShapes32[s][0], bn = kShapes32[s][1];
+    for (size_t i = 0; i < tasks.size(); ++i)
+      for (int m0 = 0; m0 < tasks[i].m; m0 += bm)
+        for (int n0 = 0; n0 < tasks[i].n; n0 += bn) nt.push_back(GemmTile{(int32_t)i, m0, n0, 0});
   }
   GemmTile* d = nullptr;
   if (!nt.empty()) {
@@ -311,44 +527,48 @@ int GemmPlan::retile(int s, cudaStream_t st) {
       return rc;
     }
   }
-  if (d_tiles) dfree(d_tiles);
-  d_tiles = d;
-  tiles.swap(nt);
-  shape = s;
+  GemmTiles& to = fp32 ? t32 : t64;
+  if (to.d) dfree(to.d);
+  to.d = d;
+  to.n = (int64_t)nt.size();
+  to.shape = s;
   return CMPS_OK;
 }
+
+int GemmPlan::tile_fp32(cudaStream_t st) { return retile(true, pick_shape32(*this), st); }
 
 namespace {
 std::mutex g_tune_mu;
 std::map<std::vector<int64_t>, int> g_tune_cache;  // plan signature -> measured best shape
 }  // namespace
 
-int autotune_plan(GemmPlan& p, int role, const std::function<int()>& run, cudaStream_t st, TuneStats* stats) {
+int autotune_plan(GemmPlan& p, int role, bool fp32, const std::function<int()>& run, cudaStream_t st,
+                  TuneStats* stats) {
   if (p.tasks.empty()) return CMPS_OK;
+  const int heuristic = (fp32 ? p.t32 : p.t64).shape;
   // signature: the role, the task and term counts, the flops to 3 digits and
-  // the padded-work choice -- plans of the same shape population share it
+  // the modelled choice -- plans of the same shape population share it
   double fl = 0.0;
   for (const GemmTask& t : p.tasks)
     for (int q = t.t0; q < t.t1; ++q) fl += 8.0 * t.m * (double)t.n * p.terms[q].k;
   const int64_t fq = fl > 0.0 ? (int64_t)std::llround(std::log10(fl) * 300.0) : 0;
-  const std::vector<int64_t> sig{role, (int64_t)p.tasks.size(), (int64_t)p.terms.size(), fq, p.shape};
+  const std::vector<int64_t> sig{role, (int64_t)p.tasks.size(), (int64_t)p.terms.size(), fq, heuristic};
   {
     std::lock_guard<std::mutex> lock(g_tune_mu);
     auto it = g_tune_cache.find(sig);
     if (it != g_tune_cache.end()) {
       if (stats) ++stats->cached;
-      return it->second == p.shape ? CMPS_OK : p.retile(it->second, st);
+      return it->second == heuristic ? CMPS_OK : p.retile(fp32, it->second, st);
     }
   }
-  const int heuristic = p.shape;
   float best = 0.0f, heur = 0.0f;
   int pick = heuristic;
   cudaEvent_t e0, e1;
   CMPS_CUDA(cudaEventCreate(&e0));
   CMPS_CUDA(cudaEventCreate(&e1));
   int rc = CMPS_OK;
-  for (int s = 0; s < 3 && rc == CMPS_OK; ++s) {
-    rc = p.retile(s, st);
+  for (int s = 0; s < (fp32 ? 3 : kNumShapes64) && rc == CMPS_OK; ++s) {
+    rc = p.retile(fp32, s, st);
     if (rc == CMPS_OK) rc = run();  // warm-up
     if (rc != CMPS_OK) break;
     cudaEventRecord(e0, st);
@@ -360,6 +580,7 @@ int autotune_plan(GemmPlan& p, int role, const std::function<int()>& run, cudaSt
     }
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e0, e1);
+    if (std::getenv("CMPS_TUNE_TRACE")) std::fprintf(stderr, "  role %d shape %d: %.4f ms\n", role, s, ms / 3);
     if (s == heuristic) heur = ms;
     if (s == 0 || ms < best) {
       best = ms;
@@ -369,7 +590,7 @@ int autotune_plan(GemmPlan& p, int role, const std::function<int()>& run, cudaSt
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
   CMPS_TRY(rc);
-  CMPS_TRY(p.retile(pick, st));
+  CMPS_TRY(p.retile(fp32, pick, st));
   if (std::getenv("CMPS_TUNE_TRACE"))
     std::fprintf(stderr, "autotune role %d: tasks %zu, heuristic shape %d %.3f ms, best shape %d %.3f ms\n", role,
                  p.tasks.size(), heuristic, heur / 3, pick, best / 3);
@@ -384,14 +605,6 @@ int autotune_plan(GemmPlan& p, int role, const std::function<int()>& run, cudaSt
 }
 
 int GemmPlan::upload(cudaStream_t st) {
-  shape = pick_shape(*this);
-  const int bm = kShapes[shape][0], bn = kShapes[shape][1];
-  tiles.clear();
-  for (size_t i = 0; i < tasks.size(); ++i) {
-    const GemmTask& t = tasks[i];
-    for (int m0 = 0; m0 < t.m; m0 += bm)
-      for (int n0 = 0; n0 < t.n; n0 += bn) tiles.push_back(GemmTile{(int32_t)i, m0, n0, 0});
-  }
   release();
   auto up = [st](auto& v, auto** d) -> int {
     if (v.empty()) return CMPS_OK;
@@ -401,8 +614,7 @@ int GemmPlan::upload(cudaStream_t st) {
   };
   CMPS_TRY(up(tasks, &d_tasks));
   CMPS_TRY(up(terms, &d_terms));
-  CMPS_TRY(up(tiles, &d_tiles));
-  return CMPS_OK;
+  return retile(false, pick_shape64(*this), st);
 }
 
 int GemmPlan::validate(bool a_h, bool b_h, int64_t a_len, int64_t b_len, int64_t c_len, const char* what) const {
@@ -439,11 +651,12 @@ int GemmPlan::validate(bool a_h, bool b_h, int64_t a_len, int64_t b_len, int64_t
 void GemmPlan::release() {
   if (d_tasks) dfree(d_tasks);
   if (d_terms) dfree(d_terms);
-  if (d_tiles) dfree(d_tiles);
   d_tasks = nullptr;
   d_terms = nullptr;
-  d_tiles = nullptr;
+  for (GemmTiles* t : {&t64, &t32}) {
+    if (t->d) dfree(t->d);
+    *t = GemmTiles{};
+  }
 }
-
 
 }  // namespace cmps

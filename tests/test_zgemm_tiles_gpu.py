@@ -1,0 +1,57 @@
+"""The grouped FP64 GEMM at the edges of its tiles: sector dimensions one off
+every slice and tile boundary (8, 16, 32, 64), K around the 16-value stage
+and the 128-value fold, tasks of a single row or column -- through both
+contraction orders, with complex and with real MPO entries (the real-A form).
+
+The forward error of a stage is at most 2 (kFold + K / kFold + 6) u times the
+product of the operands' absolute values (u = 2^-53; the factor 2 for the
+three-multiplication imaginary part), under 300 u for K up to 2000; four
+stages and the oracle's own sums stay under 1500 u of the matvec taken with
+absolute values throughout."""
+import numpy as np
+import pytest
+
+from oracle import blocks as ob
+
+pytestmark = pytest.mark.gpu
+
+U = 2.0 ** -53
+LEFT = [1, 2, 7, 8, 9, 15, 17, 31, 33, 64, 65, 129]
+RIGHT = [130, 5, 63, 32, 16, 8, 40, 1, 24, 3, 96, 10]
+
+
+def _bond(dims):
+    return np.repeat(np.arange(len(dims)), dims).reshape(-1, 1).astype(np.int64)
+
+
+def _mats(t, chi, D):
+    return ob.env_matrices(chi, D, t.colptr, t.rowind, t.values)
+
+
+@pytest.mark.parametrize("d,real_w", [(1, False), (3, False), (3, True), (17, True)])
+def test_matvec_at_tile_edges(d, real_w):
+    from chainamps_b200 import (Context, TwoVertexComponents, models, CMPS_ORDER_FOLDED, CMPS_ORDER_CANONICAL)
+    D, rules = 3, (0,)
+    rng = np.random.default_rng(d)
+    bl, br = (_bond(LEFT), _bond(RIGHT)) if d < 17 else (_bond(LEFT[:6]), _bond(RIGHT[3:9]))
+    ch, bq = np.zeros((d, 1), np.int64), np.array([[0], [1], [-1]], np.int64)
+    W = rng.standard_normal((d, D, d, D)) + (0 if real_w else 1j) * rng.standard_normal((d, D, d, D))
+    # an entry conserves charge: q(b) = q(b') as the states carry none
+    W = W * (bq[:, 0][None, :, None, None] == bq[:, 0][None, None, None, :]).astype(float)
+    W = W.astype(np.complex128)
+    L = models.random_environment(rng, rules, bl, bq, list(range(D)), right=False)
+    R = models.random_environment(rng, rules, br, bq, list(range(D)), right=True)
+    lm, rm = _mats(L, bl.shape[0], D), _mats(R, br.shape[0], D)
+    ref = ob.BlockHeff(rules, ch, bl, br, bq, W, lm, rm)
+    mag = ob.BlockHeff(rules, ch, bl, br, bq, np.abs(W).astype(np.complex128),
+                       *[[None if m is None else np.abs(m).astype(np.complex128) for m in e] for e in (lm, rm)])
+    x = rng.standard_normal(ref.n) + 1j * rng.standard_normal(ref.n)
+    want, bound = ref.matvec(x), 1500 * U * np.abs(mag.matvec(np.abs(x).astype(np.complex128)))
+    ctx = Context(0)
+    h = TwoVertexComponents(ctx, rules, L, models.mpo_tensor(ch, W, bq), R)
+    for order in (CMPS_ORDER_FOLDED, CMPS_ORDER_CANONICAL):
+        h.set_order(order)
+        err = np.abs(h.multiply(x) - want)
+        assert np.all(err <= bound), (order, np.max(err / np.maximum(bound, 1e-300)))
+    del h
+    ctx.close()

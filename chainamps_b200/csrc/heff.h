@@ -107,9 +107,11 @@ struct Heff {
   AxpyBlock* d_rp_blocks = nullptr;
   AxpyTerm* d_rp_terms = nullptr;
   std::map<std::array<int, 4>, int64_t> lp_off, rp_off;  // (b1, sigma', sigma, sector) -> offset
-  std::vector<int64_t> t_base;   // [b1 * nm + m] -> offset into T, -1 if absent
+  std::vector<int64_t> t_base;   // [b1 * nm + m] -> offset into T, -1 if no element is both produced and read
+  std::vector<std::vector<uint8_t>> t_reads;  // [b1 * nm + m][sigma2]: stage 2 reads these columns of the block
   Planar T;                      // stage-1 intermediate, allocated on first use (ensure_T)
   int64_t t_len = 0;             // its length in complex elements
+  int64_t t_full = 0;            // the same with zero rows and unread columns kept
   int ensure_T();
   GemmPlan stage1, stage2;
   // Output sectors this matvec computes (1 = owned).  All of them, unless the
@@ -157,9 +159,10 @@ struct Heff {
   // two stages above) or canonical (L, W1, W2, R one index at a time,
   // canonical.cu).  order_req is what the caller asked for (CMPS_ORDER_*),
   // order the one in use; flops_folded / flops_canon are the executed flops
-  // of each order.
+  // of each order, flops_folded_full the folded order's with T's zero rows
+  // and unread columns kept: what the choice of an order is measured by.
   int order_req = CMPS_ORDER_AUTO, order = CMPS_ORDER_FOLDED;
-  double flops_folded = 0.0, flops_canon = 0.0;
+  double flops_folded = 0.0, flops_canon = 0.0, flops_folded_full = 0.0;
   Canon* canon = nullptr;
   int select_order();
   // The split-precision operator runs the canonical order instead of the

@@ -62,7 +62,9 @@ extern "C" int cmps_heff_apply_device_noalloc(cmps_heff* h, const double* d_in, 
     return fail(CMPS_ERR_ARG, "the no-allocation matvec runs the FP64 path only; set CMPS_FP64 on the handle");
   if (H.proj_np || !H.whole())
     return fail(CMPS_ERR_ARG, "the no-allocation matvec runs the plain unsharded operator (no projectors)");
-  const int64_t need = 4 * H.th.total + 2 * H.t_len;
+  // the size limit counts T with its zero rows and unread columns, which are
+  // not stored
+  const int64_t need = 4 * H.th.total + 2 * H.t_full;
   if (need > kNoAllocScratchDoubles)
     return fail(CMPS_ERR_ARG, "no-allocation matvec: this H_eff needs " + std::to_string(need * 8) +
                                   " bytes of scratch, above the static maximum of " +

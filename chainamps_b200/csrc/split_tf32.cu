@@ -171,6 +171,19 @@ void add_tiles(TcPlan& p, int32_t task, int32_t m, int32_t n) {
       p.tiles.push_back(TcTile{task, m0, n0, b_box_rows(n), 0, ((std::min(128, n - n0)) + 15) & ~15});
 }
 
+// Tiles over the row ranges `used` only (ascending): each tile of 128 rows
+// begins at the first used row that no earlier tile covers, which needs the
+// fewest tiles.
+void add_tiles(TcPlan& p, int32_t task, const std::vector<std::pair<int32_t, int32_t>>& used, int32_t n) {
+  int32_t done = 0;  // rows before this one are covered
+  for (const auto& u : used)
+    for (int32_t m0 = std::max(u.first, done); m0 < u.second; m0 += 128) {
+      for (int32_t n0 = 0; n0 < n; n0 += 128)
+        p.tiles.push_back(TcTile{task, m0, n0, b_box_rows(n), 0, ((std::min(128, n - n0)) + 15) & ~15});
+      done = m0 + 128;
+    }
+}
+
 void mark_vector_stores(TcPlan& p, const void* out, int64_t plane) {
   for (TcTask& t : p.tasks) {
     bool ok = ((uintptr_t)out & 15) == 0 && t.row_stride == 1 && t.m % 8 == 0 && t.col_stride % 8 == 0 &&
@@ -365,6 +378,7 @@ static int build_split(Heff& H, bool bf16) {
     int32_t ntot = 0;
     std::vector<std::array<int, 4>> tk;    // stage 1: (s1, s, 0, 0); stage 2: (b1, m, s2, t)
     std::vector<Seg> segs;
+    std::vector<uint8_t> reads;            // stage 1: states sigma2 whose columns of T stage 2 reads
   };
   auto fuse = [](std::vector<std::pair<std::vector<int64_t>, std::pair<Fused, Seg>>>& raw, int32_t max_seg_n) {
     // raw: (signature, (task shape, its segment)) in creation order
@@ -396,6 +410,8 @@ static int build_split(Heff& H, bool bf16) {
         }
         cur.ntot += sg.n;
         cur.segs.push_back(std::move(sg));
+        const std::vector<uint8_t>& rd = raw[i].second.first.reads;
+        for (size_t q = 0; q < rd.size(); ++q) cur.reads[q] |= rd[q];
       }
       if (open) out.push_back(std::move(cur));
     }
@@ -424,6 +440,8 @@ static int build_split(Heff& H, bool bf16) {
             sg.keys.push_back({b1, s1p, s1, sa});
             sig.push_back(s1);
           }
+          if (sg.keys.empty()) continue;  // rows of T that stay zero from its first fill
+          shape.reads = H.t_reads[(size_t)b1 * nm + m];
           raw.push_back({sig, {shape, sg}});
         }
       }
@@ -623,7 +641,19 @@ static int build_split(Heff& H, bool bf16) {
       if (sg.out_off < 0 || sg.out_off + (int64_t)(task.m - 1) * task.row_stride + (int64_t)(sg.n - 1) * task.col_stride >=
                                 S->ts_len)
         return fail(CMPS_ERR_STATE, "stage-1 output outside TS");
-    tc::add_tiles(p1, (int32_t)p1.tasks.size(), task.m, task.n);
+    // the chunks of T's columns (here rows of C1) that stage 2 reads for some
+    // segment, in row order; the rest of T stays zero from its first fill.
+    // With the rows that no LeftPart block produces left out too, stage 1
+    // writes about half of T on the spin ladder (matvec at chi = 512 in split
+    // BF16: 1.91 -> 1.68 ms; the same bits).
+    std::vector<std::pair<int32_t, int32_t>> used;
+    for (int s2 = 0; s2 < d; ++s2)
+      if (f.reads[s2]) {
+        const int t = A2.find(r.add(th.mq[m], H.sigq[s2]));
+        used.push_back({(int32_t)S->coloff_pad[m][s2], (int32_t)(S->coloff_pad[m][s2] + S->pad(A2.sdim[t]))});
+      }
+    std::sort(used.begin(), used.end());
+    tc::add_tiles(p1, (int32_t)p1.tasks.size(), used, task.n);
     p1.tasks.push_back(task);
   }
   // ---- stage 2 plan: C2[l', a2'] = sum TS[l', r_pad] RPTS[a2', a2] ----
@@ -706,7 +736,7 @@ int prepare_precision(Heff* h, int precision) {
   if (h->split && h->split->bf16 != bf16) release_split(h);
   if (h->low_canonical && (h->ctc != nullptr) != (bf16 && h->whole())) release_split(h);
   if (h->split || h->low_canonical) return CMPS_OK;
-  if (h->canon && (h->order_req == CMPS_ORDER_CANONICAL || h->flops_canon <= kLowCanonicalRatio * h->flops_folded)) {
+  if (h->canon && (h->order_req == CMPS_ORDER_CANONICAL || h->flops_canon <= kLowCanonicalRatio * h->flops_folded_full)) {
     if (bf16 && h->whole()) {
       const int st = build_canonical_tc(*h);
       if (st == CMPS_OK) {

@@ -5,6 +5,7 @@
 #include <cuda_runtime.h>
 #include <stdint.h>
 
+#include <utility>
 #include <vector>
 
 #include "internal.h"
@@ -81,6 +82,8 @@ int encode_map(bool bf16, const void* base, int64_t K, int64_t rows, int64_t ld,
                int box_rows, CUtensorMap* out);
 // Tiles of a task of m x n outputs, 128 x 128 each (row-major over the task).
 void add_tiles(TcPlan& p, int32_t task, int32_t m, int32_t n);
+// The same over the row ranges `used` (begin, end; ascending) only.
+void add_tiles(TcPlan& p, int32_t task, const std::vector<std::pair<int32_t, int32_t>>& used, int32_t n);
 // Completes a plan built term by term: k-steps per tile, optionally the
 // heaviest tiles first, and checks every term, task, segment list and tile.
 // by_tma: the A operands are tensor maps (else converter descriptors);

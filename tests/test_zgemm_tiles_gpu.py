@@ -55,3 +55,40 @@ def test_matvec_at_tile_edges(d, real_w):
         assert np.all(err <= bound), (order, np.max(err / np.maximum(bound, 1e-300)))
     del h
     ctx.close()
+
+
+@pytest.mark.parametrize("seed", [1, 2, 3])
+def test_folded_order_skips_zero_parts_of_t(seed):
+    """Sparse MPOs in the folded order: slots that no LeftPart block produces,
+    slots that no RightPart block reads, states that a slot connects on one
+    side only, neighbouring states alike and unlike -- the rows and columns
+    of T that the plans leave out.  FP64 as above; the split forms within
+    2e-4 of the largest entry, as the other split tests at these sizes."""
+    from chainamps_b200 import (Context, TwoVertexComponents, models, CMPS_FP64, CMPS_SPLIT_TF32, CMPS_SPLIT_BF16,
+                                CMPS_ORDER_FOLDED)
+    d, D, rules = 5, 6, (0,)
+    rng = np.random.default_rng(seed)
+    bl, br = _bond([9, 33, 1, 17]), _bond([40, 8, 3, 21])
+    ch, bq = np.zeros((d, 1), np.int64), np.zeros((D, 1), np.int64)
+    W = rng.standard_normal((d, D, d, D)) + 1j * rng.standard_normal((d, D, d, D))
+    W = W * (rng.random((d, D, d, D)) < 0.06)
+    W[:, :, :, 2] = 0     # produced by nothing
+    W[:, 3] = 0           # read by nothing
+    W[0, 0, 0, 0] = 1.0   # never empty
+    L = models.random_environment(rng, rules, bl, bq, list(range(D)), right=False)
+    R = models.random_environment(rng, rules, br, bq, list(range(D)), right=True)
+    lm, rm = _mats(L, bl.shape[0], D), _mats(R, br.shape[0], D)
+    ref = ob.BlockHeff(rules, ch, bl, br, bq, W, lm, rm)
+    mag = ob.BlockHeff(rules, ch, bl, br, bq, np.abs(W).astype(np.complex128),
+                       *[[None if m is None else np.abs(m).astype(np.complex128) for m in e] for e in (lm, rm)])
+    x = rng.standard_normal(ref.n) + 1j * rng.standard_normal(ref.n)
+    want, bound = ref.matvec(x), 1500 * U * np.abs(mag.matvec(np.abs(x).astype(np.complex128)))
+    ctx = Context(0)
+    for prec in (CMPS_FP64, CMPS_SPLIT_TF32, CMPS_SPLIT_BF16):
+        h = TwoVertexComponents(ctx, rules, L, models.mpo_tensor(ch, W, bq), R)
+        h.set_order(CMPS_ORDER_FOLDED)
+        h.set_precision(prec)
+        err = np.abs(h.multiply(x) - want)
+        assert np.all(err <= (bound if prec == CMPS_FP64 else 2e-4 * np.max(np.abs(want)))), (prec, np.max(err))
+        del h
+    ctx.close()

@@ -660,12 +660,18 @@ int build_canonical_tc(Heff& H) {
     }
     // Tiles of a group of tasks that read the same A rows go row tile by row
     // tile across the group, so the tiles that run at the same time (dealt
-    // round-robin to the SMs) share their A tiles in L2.
+    // round-robin to the SMs) share their A tiles in L2.  Where the
+    // number of tasks divides 148 (4 in stage R of the Ising chains) an SM would
+    // get the same task, heavy or light, in every row tile: the tasks' order
+    // then rotates from row tile to row tile.
     for (auto& g : groups) {
       int32_t mmax = 0;
       for (int32_t t : g.second) mmax = std::max(mmax, p.tasks[t].m);
-      for (int32_t m0 = 0; m0 < mmax; m0 += 128)
-        for (int32_t t : g.second) {
+      const size_t shift = 148 % g.second.size() == 0 ? 1 : 0;
+      size_t turn = 0;
+      for (int32_t m0 = 0; m0 < mmax; m0 += 128, turn += shift)
+        for (size_t i = 0; i < g.second.size(); ++i) {
+          const int32_t t = g.second[(i + turn) % g.second.size()];
           const tc::TcTask& k = p.tasks[t];
           if (m0 >= k.m) continue;
           for (int32_t n0 = 0; n0 < k.n; n0 += 128)

@@ -130,8 +130,15 @@ __device__ __forceinline__ unsigned long long now_ns() {
   return t;
 }
 // Bounded wait (wall-clock limit): returns false, and raises *err, when the
-// limit is reached or another CTA already raised it.
+// limit is reached or another CTA already raised it.  The clock and the
+// error word are read only when the barrier has not flipped after a few
+// polls (each of which may suspend the thread for a while): most waits are for
+// barriers that have flipped already, and reading the global timer for each
+// cost 2 to 3% of a stage.
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int* err, int code) {
+#pragma unroll 1
+  for (int i = 0; i < 8; ++i)
+    if (mbar_try(bar, parity)) return true;
   const unsigned long long t0 = now_ns();
   while (!mbar_try(bar, parity)) {
     if (now_ns() - t0 > kWaitLimitNs) {
@@ -158,8 +165,12 @@ __device__ __forceinline__ void tma_load_3d(void* dst, const CUtensorMap* map, i
       : "memory");
 }
 
-__device__ __forceinline__ void sts16(uint32_t addr, uint32_t v) {
-  asm volatile("st.shared.u16 [%0], %1;" ::"r"(addr), "h"((unsigned short)v) : "memory");
+// four 8 x 8 matrices of 16-bit elements, each stored transposed: lane
+// 8 q + j gives the address of column j of matrix q, 8 rows = 16 bytes
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t addr, uint32_t a, uint32_t b, uint32_t c, uint32_t d) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(addr), "r"(a), "r"(b),
+               "r"(c), "r"(d)
+               : "memory");
 }
 
 // UMMA shared-memory descriptor, K-major, SWIZZLE_64B: 64-byte rows, 8-row
@@ -207,6 +218,17 @@ __device__ __forceinline__ void tmem_ld16_issue(uint32_t taddr, uint32_t* r) {
       : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
         "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
       : "r"(taddr));
+}
+// The same 16 columns of 32 lanes as two 16x256b loads: register 8 h + 4 g +
+// 2 u + e of lane l holds row 16 h + 8 u + l / 4, column 8 g + 2 (l % 4) + e,
+// the fragment layout that stmatrix takes.
+__device__ __forceinline__ void tmem_ld16_frag_issue(uint32_t taddr, uint32_t* r) {
+#pragma unroll
+  for (int h = 0; h < 2; ++h)
+    asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0,%1,%2,%3,%4,%5,%6,%7}, [%8];"
+                 : "=r"(r[8 * h]), "=r"(r[8 * h + 1]), "=r"(r[8 * h + 2]), "=r"(r[8 * h + 3]), "=r"(r[8 * h + 4]),
+                   "=r"(r[8 * h + 5]), "=r"(r[8 * h + 6]), "=r"(r[8 * h + 7])
+                 : "r"(taddr + ((uint32_t)(16 * h) << 16)));
 }
 // wait for the outstanding tcgen05.ld; the registers pass through the asm so
 // that no read of them moves above the wait
@@ -602,37 +624,54 @@ tc_split_gemm(const TcTile* __restrict__ tiles, int ntiles, const TcTask* __rest
       const int c_step = 16 * epi_per_quad<MODE>();
       // TMEM loads run one chunk ahead: chunk c + c_step is in flight while
       // chunk c is stored (every lane issues and waits; tcgen05.ld is
-      // warp-collective, so the row check comes after)
+      // warp-collective, so the row check comes after).
+      //
+      // Vector-store chunks (mode 3): 16 columns inside one column segment of
+      // a task that admits 16-byte stores of 8-row runs.  They are loaded in
+      // the fragment layout, split into BF16 there, transposed by stmatrix
+      // into a [plane][column][row] box in shared memory and stored from it as
+      // 16-byte runs.
+      auto segment = [&](int col) {
+        return (col >= task.seg_n0[1]) + (col >= task.seg_n0[2]) + (col >= task.seg_n0[3]);
+      };
+      auto vector_chunk = [&](int c) {
+        const int cnt = min(16, ntile - c);
+        return MODE == 3 && task.vstore && cnt > 0 && segment(tile.n0 + c) == segment(tile.n0 + c + cnt - 1);
+      };
       uint32_t ra[16], ia[16];
       const bool wide = wide_tile<MODE>(tile);
-      if (have && !wide && c_first < nmma) {
-        tmem_ld16_issue(tbase + c_first, ra);
-        tmem_ld16_issue(tbase + 128 + c_first, ia);
-      }
+      auto load_pair = [&](bool vec, uint32_t pa, uint32_t pb) {
+        if (MODE == 3 && vec) {
+          tmem_ld16_frag_issue(pa, ra);
+          tmem_ld16_frag_issue(pb, ia);
+        } else {
+          tmem_ld16_issue(pa, ra);
+          tmem_ld16_issue(pb, ia);
+        }
+      };
+      bool vec = vector_chunk(c_first);
+      if (have && !wide && c_first < nmma) load_pair(vec, tbase + c_first, tbase + 128 + c_first);
       for (int c = c_first; c < nmma; c += c_step) {
         float vr[16], vi[16];
+        const bool vec_next = c + c_step < nmma && vector_chunk(c + c_step);
         if (have && wide) {
           // four-plane form: block q of d_re / d_im (columns q N ..) holds
           // A_re . B_q / A_im . B_q for B planes re_hi, re_mid, im_hi, im_mid
           //   re = d_re[0] + d_re[1] - d_im[2] - d_im[3]
           //   im = d_re[2] + d_re[3] + d_im[0] + d_im[1]
-          tmem_ld16_issue(tbase + c, ra);
-          tmem_ld16_issue(tbase + nmma + c, ia);
+          load_pair(vec, tbase + c, tbase + nmma + c);
           tmem_wait(ra, ia);
 #pragma unroll
           for (int i = 0; i < 16; ++i) vr[i] = __uint_as_float(ra[i]) + __uint_as_float(ia[i]);
-          tmem_ld16_issue(tbase + 128 + 2 * nmma + c, ra);
-          tmem_ld16_issue(tbase + 128 + 3 * nmma + c, ia);
+          load_pair(vec, tbase + 128 + 2 * nmma + c, tbase + 128 + 3 * nmma + c);
           tmem_wait(ra, ia);
 #pragma unroll
           for (int i = 0; i < 16; ++i) vr[i] -= __uint_as_float(ra[i]) + __uint_as_float(ia[i]);
-          tmem_ld16_issue(tbase + 2 * nmma + c, ra);
-          tmem_ld16_issue(tbase + 3 * nmma + c, ia);
+          load_pair(vec, tbase + 2 * nmma + c, tbase + 3 * nmma + c);
           tmem_wait(ra, ia);
 #pragma unroll
           for (int i = 0; i < 16; ++i) vi[i] = __uint_as_float(ra[i]) + __uint_as_float(ia[i]);
-          tmem_ld16_issue(tbase + 128 + c, ra);
-          tmem_ld16_issue(tbase + 128 + nmma + c, ia);
+          load_pair(vec, tbase + 128 + c, tbase + 128 + nmma + c);
           tmem_wait(ra, ia);
 #pragma unroll
           for (int i = 0; i < 16; ++i) vi[i] += __uint_as_float(ra[i]) + __uint_as_float(ia[i]);
@@ -643,67 +682,68 @@ tc_split_gemm(const TcTile* __restrict__ tiles, int ntiles, const TcTask* __rest
             vr[i] = __uint_as_float(ra[i]);
             vi[i] = __uint_as_float(ia[i]);
           }
-          if (c + c_step < nmma) {
-            tmem_ld16_issue(tbase + c + c_step, ra);
-            tmem_ld16_issue(tbase + 128 + c + c_step, ia);
-          }
+          if (c + c_step < nmma) load_pair(vec_next, tbase + c + c_step, tbase + 128 + c + c_step);
         } else {
 #pragma unroll
           for (int i = 0; i < 16; ++i) vr[i] = vi[i] = 0.f;
         }
-        if (MODE == 3 && task.vstore) {
-          // Vector-store path, for a chunk inside one column segment: the
-          // chunk is split and written by every lane as its row of a
-          // [plane][column][row] box in shared memory, then read back as
-          // 16-byte runs of 8 rows and stored: lane l takes columns l / 4
-          // and 8 + l / 4, rows 8 (l % 4) .. +7, in the four planes.  Rows
-          // past the task (whole 8-row runs: its M is a multiple of 8) are
-          // not stored.
+        const bool vec_now = vec;
+        vec = vec_next;
+        if (MODE == 3 && vec_now) {
           const int cnt = min(16, ntile - c);
-          const int colA = tile.n0 + c, colB = colA + cnt - 1;
-          const int qa = (colA >= task.seg_n0[1]) + (colA >= task.seg_n0[2]) + (colA >= task.seg_n0[3]);
-          const int qb = (colB >= task.seg_n0[1]) + (colB >= task.seg_n0[2]) + (colB >= task.seg_n0[3]);
+          const int colA = tile.n0 + c, qa = segment(colA);
           const int row0 = tile.m0 + quad * 32;
-          if (cnt > 0 && qa == qb && row0 < task.m) {
-            const int n0 = qa == 0 ? 0 : qa == 1 ? task.seg_n0[1] : qa == 2 ? task.seg_n0[2] : task.seg_n0[3];
-            const int64_t so = qa == 0 ? task.seg_off[0] : qa == 1 ? task.seg_off[1] : qa == 2 ? task.seg_off[2]
-                                                                                            : task.seg_off[3];
-            const int lc = lane >> 2, lr = (lane & 3) * 8;
-            const bool rok8 = row0 + lr < task.m;
-            uint16_t* g = reinterpret_cast<uint16_t*>(out32) + so + row0 + lr +
-                          (int64_t)(colA - n0 + lc) * task.col_stride;
-            const uint32_t box = stg + (uint32_t)(lane * 2);
-            const uint32_t rd = stg + (uint32_t)(lc * 64 + lr * 2);
-            __syncwarp();  // the previous chunk's reads of the box are done
+          if (row0 >= task.m) continue;
+          const int n0 = qa == 0 ? 0 : qa == 1 ? task.seg_n0[1] : qa == 2 ? task.seg_n0[2] : task.seg_n0[3];
+          const int64_t so = qa == 0 ? task.seg_off[0] : qa == 1 ? task.seg_off[1] : qa == 2 ? task.seg_off[2]
+                                                                                          : task.seg_off[3];
+          // Box: column i of plane p at (16 p + i) 64 bytes, its four runs of
+          // 8 rows XORed by (i / 2) % 4, so that neither the transposing
+          // stores nor the 16-byte reads meet bank conflicts.  Lane l stores
+          // column l % 8 of run l / 8 and reads run l % 4 of columns l / 4 and
+          // 8 + l / 4.
+          const int sj = lane & 7, sq = lane >> 3;
+          const uint32_t wr = stg + (uint32_t)(sj * 64 + ((sq ^ (sj >> 1)) << 4));
+          const int lc = lane >> 2, lr = lane & 3;
+          const uint32_t rd = stg + (uint32_t)(lc * 64 + ((lr ^ ((lc >> 1) & 3)) << 4));
+          const bool rok8 = row0 + 8 * lr < task.m;
+          uint16_t* g = reinterpret_cast<uint16_t*>(out32) + so + row0 + 8 * lr +
+                        (int64_t)(colA - n0 + lc) * task.col_stride;
+          __syncwarp();  // the previous chunk's reads of the box are done
 #pragma unroll
-            for (int i = 0; i < 16; ++i) {
-              const float xr = vr[i], xi = vi[i];
-              const uint32_t h2 = bf16x2(xi, xr);
-              const float rh = __uint_as_float(h2 << 16), ih = __uint_as_float(h2 & 0xffff0000u);
-              const uint32_t m2 = bf16x2(xi - ih, xr - rh);
-              sts16(box + (uint32_t)((0 * 16 + i) * 64), h2);
-              sts16(box + (uint32_t)((1 * 16 + i) * 64), m2);
-              sts16(box + (uint32_t)((2 * 16 + i) * 64), h2 >> 16);
-              sts16(box + (uint32_t)((3 * 16 + i) * 64), m2 >> 16);
+          for (int gq = 0; gq < 2; ++gq) {
+            uint32_t rh[4], rm[4], ih[4], im[4];
+#pragma unroll
+            for (int k = 0; k < 4; ++k) {  // run k = 2 h + u
+              const int q = 8 * (k >> 1) + 4 * gq + 2 * (k & 1);
+              rh[k] = bf16x2(vr[q + 1], vr[q]);
+              rm[k] = bf16x2(vr[q + 1] - __uint_as_float(rh[k] & 0xffff0000u), vr[q] - __uint_as_float(rh[k] << 16));
+              ih[k] = bf16x2(vi[q + 1], vi[q]);
+              im[k] = bf16x2(vi[q + 1] - __uint_as_float(ih[k] & 0xffff0000u), vi[q] - __uint_as_float(ih[k] << 16));
             }
-            __syncwarp();
-            uint4 v[2][4];
-#pragma unroll
-            for (int h = 0; h < 2; ++h)
-#pragma unroll
-              for (int j = 0; j < 4; ++j)
-                asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
-                             : "=r"(v[h][j].x), "=r"(v[h][j].y), "=r"(v[h][j].z), "=r"(v[h][j].w)
-                             : "r"(rd + (uint32_t)((j * 16 + h * 8) * 64)));
-#pragma unroll
-            for (int h = 0; h < 2; ++h) {
-              if (!rok8 || h * 8 + lc >= cnt) continue;
-              uint16_t* gh = g + (int64_t)(h * 8) * task.col_stride;
-#pragma unroll
-              for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(gh + j * out32_plane) = v[h][j];
-            }
-            continue;
+            const uint32_t w = wr + (uint32_t)(gq * 8 * 64);
+            stmatrix_x4_trans(w, rh[0], rh[1], rh[2], rh[3]);
+            stmatrix_x4_trans(w + 1 * 16 * 64, rm[0], rm[1], rm[2], rm[3]);
+            stmatrix_x4_trans(w + 2 * 16 * 64, ih[0], ih[1], ih[2], ih[3]);
+            stmatrix_x4_trans(w + 3 * 16 * 64, im[0], im[1], im[2], im[3]);
           }
+          __syncwarp();
+          uint4 v[2][4];
+#pragma unroll
+          for (int h = 0; h < 2; ++h)
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];"
+                           : "=r"(v[h][j].x), "=r"(v[h][j].y), "=r"(v[h][j].z), "=r"(v[h][j].w)
+                           : "r"(rd + (uint32_t)((j * 16 + h * 8) * 64)));
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            if (!rok8 || h * 8 + lc >= cnt) continue;
+            uint16_t* gh = g + (int64_t)(h * 8) * task.col_stride;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) *reinterpret_cast<uint4*>(gh + j * out32_plane) = v[h][j];
+          }
+          continue;
         }
         if (!row_ok) continue;
         if (MODE == 3) {

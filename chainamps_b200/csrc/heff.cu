@@ -770,7 +770,7 @@ int Heff::finish() {
   CMPS_TRY(x.alloc(th.total));
   CMPS_TRY(y.alloc(th.total));
   CMPS_CUDA(dmalloc(&d_io, sizeof(double) * 2 * std::max<int64_t>(1, n_allowed)));
-  CMPS_TRY(ops.init(th.total));
+  CMPS_TRY(ops.init(th.total, st));
   bt.mark("work vectors");
   CMPS_TRY(select_order());
   CMPS_CUDA(cudaStreamSynchronize(st));
@@ -854,6 +854,13 @@ int Heff::build_plans() {
   // moved 2.1 x the bytes and did 1.25 x the work: 9.6 ms, now 7.9 ms (FP64).
   std::vector<int> by_off;  // states in the order of theta's rows and columns (class by class)
   for (const std::vector<int>& c : cls_mem) by_off.insert(by_off.end(), c.begin(), c.end());
+  // sector of a0 / a2 that a state of a theta row / column carries, -1 if none
+  std::vector<int> rsec((size_t)nm * d, -1), csec = rsec;
+  for (int m = 0; m < nm; ++m)
+    for (int q = 0; q < d; ++q) {
+      if (th.rowoff[m][q] >= 0) rsec[(size_t)m * d + q] = A0.find(r.sub(th.mq[m], sigq[q]));
+      if (th.coloff[m][q] >= 0) csec[(size_t)m * d + q] = A2.find(r.add(th.mq[m], sigq[q]));
+    }
   std::set<int> b1s;
   for (auto& kv2 : lp_off) b1s.insert(kv2.first[0]);
   std::set<int> b1r;
@@ -880,31 +887,32 @@ int Heff::build_plans() {
       B.col.assign(d, -1);
       double k_dim = 0.0;
       for (int s1p : by_off) {
-        if (th.rowoff[mp][s1p] < 0) continue;
+        const int sp = rsec[(size_t)mp * d + s1p];
+        if (sp < 0) continue;
         bool live = false;
         for (int s1 = 0; s1 < d; ++s1) {
-          if (th.rowoff[m][s1] < 0) continue;
-          const int s = A0.find(r.sub(th.mq[m], sigq[s1]));
-          if (lp_at(b1, s1p, s1, s) < 0) continue;
+          const int s = rsec[(size_t)m * d + s1];
+          if (s < 0 || lp_at(b1, s1p, s1, s) < 0) continue;
           live = true;
-          k_dim += (double)A0.sdim[A0.find(r.sub(th.mq[mp], sigq[s1p]))] * A0.sdim[s];
+          k_dim += (double)A0.sdim[sp] * A0.sdim[s];
         }
         if (!live) continue;
         B.row[s1p] = B.rows;
-        B.rows += A0.sdim[A0.find(r.sub(th.mq[mp], sigq[s1p]))];
+        B.rows += A0.sdim[sp];
       }
       if (!B.rows) continue;
       in_need[m] = 1;
       t_full += th.nrows[mp] * th.ncols[m];
       flops_folded_full += 8.0 * k_dim * (double)th.ncols[m];
       for (int s2 : by_off) {
-        if (th.coloff[m][s2] < 0) continue;
-        const int t = A2.find(r.add(th.mq[m], sigq[s2]));
+        const int t = csec[(size_t)m * d + s2];
+        if (t < 0) continue;
         bool read = false;
         for (int s2p = 0; s2p < d; ++s2p) {
-          if (th.coloff[mp][s2p] < 0 || rp_at(b1, s2, s2p, t) < 0) continue;
+          const int tp = csec[(size_t)mp * d + s2p];
+          if (tp < 0 || rp_at(b1, s2, s2p, t) < 0) continue;
           read = true;
-          flops_folded_full += 8.0 * (double)th.nrows[mp] * A2.sdim[t] * (double)A2.sdim[A2.find(r.add(th.mq[mp], sigq[s2p]))];
+          flops_folded_full += 8.0 * (double)th.nrows[mp] * A2.sdim[t] * (double)A2.sdim[tp];
         }
         if (!read) continue;
         B.col[s2] = B.cols;
@@ -918,7 +926,7 @@ int Heff::build_plans() {
       for (int s2 = 0; s2 < d; ++s2) rd.push_back(B.col[s2] >= 0);
       for (int s1p : by_off) {
         if (B.row[s1p] < 0) continue;
-        const int sp = A0.find(r.sub(th.mq[mp], sigq[s1p]));
+        const int sp = rsec[(size_t)mp * d + s1p];
         for (size_t i = 0; i < by_off.size();) {
           const int s2 = by_off[i];
           if (B.col[s2] < 0) {
@@ -927,7 +935,7 @@ int Heff::build_plans() {
           }
           int64_t n = 0;
           for (; i < by_off.size() && B.col[by_off[i]] == B.col[s2] + n && th.coloff[m][by_off[i]] == th.coloff[m][s2] + n; ++i)
-            n += A2.sdim[A2.find(r.add(th.mq[m], sigq[by_off[i]]))];
+            n += A2.sdim[csec[(size_t)m * d + by_off[i]]];
           GemmTask task{};
           task.c_off = t_total + B.row[s1p] * B.cols + B.col[s2];
           task.m = (int32_t)A0.sdim[sp];
@@ -935,9 +943,8 @@ int Heff::build_plans() {
           task.ldc = (int32_t)B.cols;
           task.t0 = (int32_t)stage1.terms.size();
           for (int s1 = 0; s1 < d; ++s1) {
-            if (th.rowoff[m][s1] < 0) continue;
-            int s = A0.find(r.sub(th.mq[m], sigq[s1]));
-            const int64_t lo = lp_at(b1, s1p, s1, s);
+            const int s = rsec[(size_t)m * d + s1];
+            const int64_t lo = s < 0 ? -1 : lp_at(b1, s1p, s1, s);
             if (lo < 0) continue;
             GemmTerm tm{};
             tm.a_off = lo;
@@ -984,11 +991,11 @@ int Heff::build_plans() {
         bool same = true;
         for (int b1 = 0; b1 < D && same; ++b1) same = (live_row(b1, s1p) < 0) == (live_row(b1, first) < 0);
         if (!same) break;
-        rows += A0.sdim[A0.find(r.sub(th.mq[mp], sigq[s1p]))];
+        rows += A0.sdim[rsec[(size_t)mp * d + s1p]];
       }
       for (int s2p = 0; s2p < d; ++s2p) {
-        if (th.coloff[mp][s2p] < 0) continue;
-        int tp = A2.find(r.add(th.mq[mp], sigq[s2p]));
+        const int tp = csec[(size_t)mp * d + s2p];
+        if (tp < 0) continue;
         GemmTask task{};
         task.c_off = out_base[mp] + th.rowoff[mp][first] * th.ncols[mp] + th.coloff[mp][s2p];
         task.m = (int32_t)rows;
@@ -1001,9 +1008,8 @@ int Heff::build_plans() {
           const int m = mof[b1];
           const TBlock& B = tb[(size_t)b1 * nm + m];
           for (int s2 = 0; s2 < d; ++s2) {
-            if (th.coloff[m][s2] < 0) continue;
-            int t = A2.find(r.add(th.mq[m], sigq[s2]));
-            const int64_t ro = rp_at(b1, s2, s2p, t);
+            const int t = csec[(size_t)m * d + s2];
+            const int64_t ro = t < 0 ? -1 : rp_at(b1, s2, s2p, t);
             if (ro < 0) continue;
             GemmTerm tm{};
             tm.a_off = t_base[(size_t)b1 * nm + m] + row * B.cols + B.col[s2];
@@ -1346,6 +1352,11 @@ static void tridiag_lowest(int k, const double* a, const double* b, double* lam,
   y = z;
 }
 
+// Vectors up to this length run one Lanczos step ahead of the host.  The step
+// that a cycle's end wastes costs as much as the host's turns of about 15
+// steps at 1M entries (matvec and passes 0.5 to 0.8 ms, a turn 40 to 60 us).
+constexpr int64_t kStepAhead = int64_t(1) << 20;
+
 // Restarted Lanczos with full re-orthogonalisation (the local three-term
 // step, then one classical Gram-Schmidt pass against the whole basis),
 // coefficients kept on the device and a convergence check after every step.
@@ -1376,7 +1387,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     CMPS_TRY(kv.alloc((int64_t)kdim * n));
     kv_dim = kdim;
   }
-  if (!h_ab) CMPS_CUDA(cudaMallocHost(&h_ab, sizeof(double) * 4));
+  if (!h_ab) CMPS_CUDA(cudaMallocHost(&h_ab, sizeof(double) * 8));
   const int64_t ldv = 2 * n;
   auto vre = [&](int j) { return kv.d + (int64_t)j * ldv; };
   auto view = [&](int j) {
@@ -1385,23 +1396,20 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     p.len = n;
     return p;
   };
-  double* hA = ops.d_coef;        // 2 * 129
-  double* hB = hA + 260;          // 2 * 129
-  double* nrm = hA + 520;
-  double* alpha_d = hA + 528;     // 128
-  double* beta_d = hA + 656;      // 128
-  double* scale_d = hA + 784;
+  double* nrm = ops.d_coef + 900;  // clear of the Lanczos coefficients
   eig_stats = EigStats{};
-  cudaEvent_t ev[4] = {nullptr, nullptr, nullptr, nullptr};
+  // per step in flight (two at most): matvec begin and end, step done; and the
+  // whole solve
+  cudaEvent_t ev[8] = {};
   struct EvGuard {
     cudaEvent_t* e;
     ~EvGuard() {
-      for (int i = 0; i < 4; ++i)
+      for (int i = 0; i < 8; ++i)
         if (e[i]) cudaEventDestroy(e[i]);
     }
   } ev_guard{ev};
   for (auto& e : ev) CMPS_CUDA(cudaEventCreate(&e));
-  CMPS_CUDA(cudaEventRecord(ev[2], st));
+  CMPS_CUDA(cudaEventRecord(ev[6], st));
   // start vector into x
   if (guess) {
     CMPS_CUDA(cudaMemcpyAsync(d_io, guess, sizeof(double) * 2 * n_allowed, cudaMemcpyHostToDevice, st));
@@ -1413,6 +1421,8 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
   if (!have_start || !(nrm0 > 1e-300)) CMPS_TRY(ops.random(x.re(), x.im(), 0x5eed1234ULL, st));
   CMPS_TRY(ops.mdot_dev(nullptr, nullptr, 0, 0, x.re(), x.im(), nrm, st));
   CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, true, x.re(), x.im(), st));
+  h_ab[4] = 1.0;  // a cycle's first basis vector is normalised
+  CMPS_CUDA(cudaMemcpyAsync(ops.lanczos_coef().scale, h_ab + 4, sizeof(double), cudaMemcpyHostToDevice, st));
 
   const bool mixed = is_split(precision);
   if (mixed) CMPS_TRY(split_reset_error(*this, st));
@@ -1439,34 +1449,38 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     int k = 0;
     double beta0 = -1.0;
     bool split_used = false;
-    for (int j = 0; j < kdim; ++j) {
-      const bool fp64 = all_fp64 || j == 0;
+    // Step j: y = H U_j, then the three passes of VecOps::lanczos.  The last
+    // step's vector is not part of the basis (x is free until the cycle ends).
+    auto issue = [&](int j) -> int {
+      cudaEvent_t* e = ev + 3 * (j & 1);
       Planar vj = view(j);
-      CMPS_CUDA(cudaEventRecord(ev[0], st));
-      if (fp64) {
+      CMPS_CUDA(cudaEventRecord(e[0], st));
+      if (all_fp64 || j == 0) {
         CMPS_TRY(apply_theta_fp64(vj, y, st));
       } else {
         CMPS_TRY(apply_split_async(*this, vj, y, st));
         split_used = true;
       }
-      CMPS_CUDA(cudaEventRecord(ev[1], st));
+      CMPS_CUDA(cudaEventRecord(e[1], st));
+      double* out = j + 1 < kdim ? vre(j + 1) : x.re();
+      CMPS_TRY(ops.lanczos(kv.d, ldv, y.re(), y.im(), j, out, out + n, h_ab + 2 * (j & 1), st));
+      CMPS_CUDA(cudaEventRecord(e[2], st));
+      return CMPS_OK;
+    };
+    int issued = 0;
+    for (int j = 0; j < kdim; ++j) {
+      const bool fp64 = all_fp64 || j == 0;
+      // Short vectors: the next step is issued before this one's coefficients
+      // are read (it needs them on the device only), so that the GPU does not
+      // wait for the host's turn, 40 us or so.  A cycle that ends at this step
+      // drops the extra one: its vector lies past the basis.
+      const int upto = n <= kStepAhead && (all_fp64 || j > 0) ? std::min(j + 1, kdim - 1) : j;
+      while (issued <= upto) CMPS_TRY(issue(issued++));
+      cudaEvent_t* e = ev + 3 * (j & 1);
+      CMPS_CUDA(cudaEventSynchronize(e[2]));
       ++nmv;
-      // local three-term step (y -= beta_{j-1} v_{j-1}, alpha = <v_j, y>,
-      // y -= alpha v_j), then one full classical Gram-Schmidt pass against
-      // v_0..v_j that removes what rounding and the split operator's
-      // non-Hermitian error leave behind
-      const double* vp = j > 0 ? vre(j - 1) : nullptr;
-      CMPS_TRY(ops.axpy_dot_dev(vp, vp ? vp + n : nullptr, beta_d + (j > 0 ? j - 1 : 0), vre(j), vre(j) + n, y.re(),
-                                y.im(), hA, st));
-      CMPS_TRY(ops.update_mdot_dev(hA, vre(j), vre(j) + n, kv.d, kv.d + n, ldv, j + 1, y.re(), y.im(), hB, st));
-      CMPS_TRY(ops.maxpy_norm_dev(kv.d, kv.d + n, ldv, j + 1, hB, y.re(), y.im(), nrm, st));
-      CMPS_TRY(ops.lanczos_coef(hA, hB + 2 * j, nrm, j, alpha_d, beta_d, scale_d, st));
-      if (j + 1 < kdim) CMPS_TRY(ops.scale_dev(y.re(), y.im(), scale_d, false, vre(j + 1), vre(j + 1) + n, st));
-      CMPS_CUDA(cudaMemcpyAsync(h_ab, alpha_d + j, sizeof(double), cudaMemcpyDeviceToHost, st));
-      CMPS_CUDA(cudaMemcpyAsync(h_ab + 1, beta_d + j, sizeof(double), cudaMemcpyDeviceToHost, st));
-      CMPS_CUDA(cudaStreamSynchronize(st));
       float mv_ms = 0.f;
-      CMPS_CUDA(cudaEventElapsedTime(&mv_ms, ev[0], ev[1]));
+      CMPS_CUDA(cudaEventElapsedTime(&mv_ms, e[0], e[1]));
       if (fp64) {
         ++eig_stats.mv_fp64;
         eig_stats.ms_fp64 += mv_ms;
@@ -1474,7 +1488,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
         ++eig_stats.mv_split;
         eig_stats.ms_split += mv_ms;
       }
-      const double a = h_ab[0], b = h_ab[1];
+      const double a = h_ab[2 * (j & 1)], b = h_ab[2 * (j & 1) + 1];
       al.push_back(a);
       be.push_back(b);
       k = j + 1;
@@ -1513,12 +1527,14 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     }
     if (split_used) CMPS_TRY(split_error(*this));
     if (converged && !all_fp64 && k == 1) break;
-    // Ritz vector x = sum_j y_j v_j, normalised
+    // Ritz vector x = sum_j y_j V_j, V_j = U_j / beta_{j-1}, normalised
+    for (int j = 1; j < k; ++j)
+      ycoef[j] *= be[j - 1] > 1e-14 * std::max(1.0, std::fabs(al[j - 1])) ? 1.0 / be[j - 1] : 0.0;
     CMPS_TRY(ops.combine(kv.d, kv.d + n, ldv, k, ycoef.data(), x.re(), x.im(), st));
     CMPS_TRY(ops.mdot_dev(nullptr, nullptr, 0, 0, x.re(), x.im(), nrm, st));
     CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, true, x.re(), x.im(), st));
   }
-  CMPS_CUDA(cudaEventRecord(ev[3], st));
+  CMPS_CUDA(cudaEventRecord(ev[7], st));
   // HED post-processing (DMRG_routines.cpp:870-889)
   double mx2 = 0.0;
   int64_t imx = 0;
@@ -1540,7 +1556,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
   }
   CMPS_CUDA(cudaStreamSynchronize(st));
   float total_ms = 0.f;
-  CMPS_CUDA(cudaEventElapsedTime(&total_ms, ev[2], ev[3]));
+  CMPS_CUDA(cudaEventElapsedTime(&total_ms, ev[6], ev[7]));
   eig_stats.ms_total = total_ms;
   *eval = lam;
   if (matvecs) *matvecs = nmv;

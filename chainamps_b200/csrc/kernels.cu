@@ -225,12 +225,9 @@ __device__ __forceinline__ double warp_sum(double v) {
 
 // partial[r][blk]: r = 2j, 2j+1 -> <V_j, w> (re, im) for j < k; r = 2k -> |w|^2.
 // One pass over w (held in registers per tile) and one over each V_j.
-// With `uc` set, w -= c u (c = uc[0] + i uc[1], u = (ur, ui)) first, written
-// back, and the products are taken with the updated w.
 __global__ void __launch_bounds__(KR_THREADS)
-k_mdot(const double* __restrict__ Vr, const double* __restrict__ Vi, int64_t ldv, int k, double* __restrict__ wr,
-       double* __restrict__ wi, int64_t n, const double* __restrict__ uc, const double* __restrict__ ur,
-       const double* __restrict__ ui, double* __restrict__ partial) {
+k_mdot(const double* __restrict__ Vr, const double* __restrict__ Vi, int64_t ldv, int k,
+       const double* __restrict__ wr, const double* __restrict__ wi, int64_t n, double* __restrict__ partial) {
   extern __shared__ double acc[];  // [warps][2k + 1], one row per warp: no shared-memory atomics
   const int nw = KR_THREADS / 32, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rows = 2 * k + 1;
@@ -245,13 +242,6 @@ k_mdot(const double* __restrict__ Vr, const double* __restrict__ Vi, int64_t ldv
       const int64_t i = base + (int64_t)e * KR_THREADS + threadIdx.x;
       xr[e] = i < n ? wr[i] : 0.0;
       xi[e] = i < n ? wi[i] : 0.0;
-      if (uc && i < n) {
-        const double cr = uc[0], ci = uc[1], a = ur[i], b = ui[i];
-        xr[e] -= cr * a - ci * b;
-        xi[e] -= cr * b + ci * a;
-        wr[i] = xr[e];
-        wi[i] = xi[e];
-      }
       s += xr[e] * xr[e] + xi[e] * xi[e];
     }
     s = warp_sum(s);
@@ -319,26 +309,96 @@ k_maxpy_norm(const double* __restrict__ Vr, const double* __restrict__ Vi, int64
   }
 }
 
-// Local Lanczos step: w -= beta v_prev (beta = *pb, skipped when v_prev is
-// null), then partial[0|1][blk] = <v, w> (re | im) over this CTA's elements.
-__global__ void __launch_bounds__(KR_THREADS)
-k_axpy_dot(const double* __restrict__ pr, const double* __restrict__ pi, const double* __restrict__ pb,
-           const double* __restrict__ vr, const double* __restrict__ vi, double* __restrict__ wr,
-           double* __restrict__ wi, int64_t n, double* __restrict__ partial) {
+// ---- One Lanczos step in three passes ---------------------------------------
+// The basis is kept unnormalised: vector i is U_i = V_i / s_i with the scale
+// s_i = 1 / |U_i| on the device (LanczosCoef::scale), so that no pass only
+// rescales.  With y = H U_j and w = s_j y,
+//   dot     a = <V_j, w>
+//   mdot    w' = w - beta_{j-1} V_{j-1} - a V_j;  h_i = <V_i, w'>, i <= j
+//   update  U_{j+1} = w' - sum_i h_i V_i;  beta_j = |U_{j+1}|, alpha_j = a + h_j
+// w' is formed again in `update` from the same operands by the same
+// operations (local_step: explicit fused multiply-adds), so it is never
+// stored.  Per step the passes read 2 + (j + 2) + (j + 2) vectors and write
+// one: 16 (2 j + 7) n bytes.
+// These passes are bound by HBM.  Each CTA works on tiles of 512 P elements in
+// 16-byte loads (8-byte ones where n is odd and the imaginary plane starts
+// between two 16-byte boundaries), eight of them in flight per thread and
+// vector; `mdot` keeps one partial sum per thread and vector in shared memory,
+// because a warp reduction per tile and vector took as long as the loads.
+// The partial sums are added by the last CTA to finish, in a fixed order.
+// Before (five passes, 8-byte loads): 3.0 to 4.2 TB/s of 16 (2 j + 13) n bytes,
+// 90 ms of a ladder step at chi = 512 and 121 ms of an Ising step at chi = 64;
+// now 4.7 to 5.1 TB/s of fewer bytes, 54 and 75 ms.
+template <bool V2>
+__device__ __forceinline__ double2 load2(const double* __restrict__ p, int64_t i, int64_t n) {
+  if (V2) return i < n ? *reinterpret_cast<const double2*>(p + i) : double2{0.0, 0.0};
+  return double2{i < n ? p[i] : 0.0, i + 1 < n ? p[i + 1] : 0.0};
+}
+template <bool V2>
+__device__ __forceinline__ void store2(double* __restrict__ p, int64_t i, int64_t n, double2 v) {
+  if (V2) {
+    if (i < n) *reinterpret_cast<double2*>(p + i) = v;
+  } else {
+    if (i < n) p[i] = v.x;
+    if (i + 1 < n) p[i + 1] = v.y;
+  }
+}
+
+// x + i y of one element: w' = s y - b p - (ar + i ai) v
+__device__ __forceinline__ void local_step(double& xr, double& xi, double s, double b, double pr, double pi, double ar,
+                                           double ai, double vr, double vi) {
+  xr = __fma_rn(-b, pr, __dmul_rn(s, xr));
+  xi = __fma_rn(-b, pi, __dmul_rn(s, xi));
+  xr = __fma_rn(ai, vi, __fma_rn(-ar, vr, xr));
+  xi = __fma_rn(-ai, vr, __fma_rn(-ar, vi, xi));
+}
+
+// The rows of partial sums of a launch (partial[row][CTA]), added up by the
+// CTA that finishes last; true in its threads, with out[row] visible to them.
+__device__ __forceinline__ bool add_partials(const double* __restrict__ partial, int rows, double* __restrict__ out,
+                                             unsigned* __restrict__ count) {
+  __shared__ bool last;
+  __threadfence();
+  __syncthreads();
+  if (threadIdx.x == 0) last = atomicAdd(count, 1u) == gridDim.x - 1;
+  __syncthreads();
+  if (!last) return false;
+  __threadfence();
+  for (int r = threadIdx.x >> 5; r < rows; r += KR_THREADS / 32) {
+    double s = 0.0;
+    for (int b = threadIdx.x & 31; b < (int)gridDim.x; b += 32) s += __ldcg(partial + (int64_t)r * gridDim.x + b);
+    s = warp_sum(s);
+    if ((threadIdx.x & 31) == 0) out[r] = s;
+  }
+  if (threadIdx.x == 0) *count = 0u;  // for the next launch on the stream
+  __syncthreads();
+  return true;
+}
+
+// a = s_j^2 <U_j, y>
+template <bool V2, int P>
+__global__ void __launch_bounds__(KR_THREADS, 2)
+k_lanczos_dot(const double* __restrict__ ur, const double* __restrict__ ui, const double* __restrict__ yr,
+              const double* __restrict__ yi, int64_t n, int j, LanczosCoef c, double* __restrict__ partial,
+              unsigned* __restrict__ count) {
   __shared__ double red[2][KR_THREADS / 32];
-  const double b = pr ? *pb : 0.0;
   double sr = 0.0, si = 0.0;
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double xr = wr[i], xi = wi[i];
-    if (pr) {
-      xr -= b * pr[i];
-      xi -= b * pi[i];
-      wr[i] = xr;
-      wi[i] = xi;
+  const int64_t tile = (int64_t)KR_THREADS * 2 * P;
+  for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
+    double2 a[P], b[P], x[P], y[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int64_t i = base + (int64_t)(p * KR_THREADS + threadIdx.x) * 2;
+      a[p] = load2<V2>(ur, i, n);
+      b[p] = load2<V2>(ui, i, n);
+      x[p] = load2<V2>(yr, i, n);
+      y[p] = load2<V2>(yi, i, n);
     }
-    const double ar = vr[i], ai = vi[i];
-    sr += ar * xr + ai * xi;
-    si += ar * xi - ai * xr;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      sr += a[p].x * x[p].x + b[p].x * y[p].x + a[p].y * x[p].y + b[p].y * y[p].y;
+      si += a[p].x * y[p].x - b[p].x * x[p].x + a[p].y * y[p].y - b[p].y * x[p].y;
+    }
   }
   sr = warp_sum(sr);
   si = warp_sum(si);
@@ -352,20 +412,160 @@ k_axpy_dot(const double* __restrict__ pr, const double* __restrict__ pi, const d
     for (int w = 0; w < KR_THREADS / 32; ++w) t += red[threadIdx.x][w];
     partial[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
   }
+  if (add_partials(partial, 2, c.a, count) && threadIdx.x < 2) c.a[threadIdx.x] *= c.scale[j] * c.scale[j];
 }
 
-// Lanczos coefficients of step j: alpha_j = *a1 + *a2 (the real parts of the
-// two projections on v_j), beta_j = |w|; scale = 1 / beta_j, or 0 when the
-// Krylov space is exhausted (the next basis vector is then zero).
-__global__ void k_lanczos_coef(const double* __restrict__ a1, const double* __restrict__ a2,
-                               const double* __restrict__ nrm2, int j, double* __restrict__ alpha,
-                               double* __restrict__ beta, double* __restrict__ scale) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  const double a = *a1 + *a2;
-  const double b = sqrt(fmax(0.0, *nrm2));
-  alpha[j] = a;
-  beta[j] = b;
-  *scale = b > 1e-14 * fmax(1.0, fabs(a)) ? 1.0 / b : 0.0;
+// h_i = s_i <U_i, w'> for c0 <= i < c1; U_i at U + i ldv (re; im n further)
+template <bool V2, int P>
+__global__ void __launch_bounds__(KR_THREADS, 2)
+k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restrict__ yr,
+               const double* __restrict__ yi, int64_t n, int j, int c0, int c1, LanczosCoef c,
+               double* __restrict__ partial, unsigned* __restrict__ count) {
+  extern __shared__ double2 dots[];  // [c1 - c0][KR_THREADS]
+  const int tid = threadIdx.x;
+  for (int i = 0; i < c1 - c0; ++i) dots[i * KR_THREADS + tid] = double2{0.0, 0.0};
+  const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
+  const double ar = c.a[0] * s, ai = c.a[1] * s;
+  const double* uj = U + (int64_t)j * ldv;
+  const double* up = j > 0 ? uj - ldv : uj;
+  const int64_t tile = (int64_t)KR_THREADS * 2 * P;
+  for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
+    double2 x[P], y[P];
+    const int64_t i0 = base + (int64_t)tid * 2;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+      x[p] = load2<V2>(yr, i, n);
+      y[p] = load2<V2>(yi, i, n);
+    }
+    double2 v[P], u[P];
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+      v[p] = load2<V2>(uj, i, n);
+      u[p] = load2<V2>(uj + n, i, n);
+      const double2 pr = load2<V2>(up, i, n), pi = load2<V2>(up + n, i, n);
+      local_step(x[p].x, y[p].x, s, b, pr.x, pi.x, ar, ai, v[p].x, u[p].x);
+      local_step(x[p].y, y[p].y, s, b, pr.y, pi.y, ar, ai, v[p].y, u[p].y);
+    }
+#pragma unroll 2
+    for (int q = c0; q < c1; ++q) {
+      const double* vq = U + (int64_t)q * ldv;
+      double2 t{0.0, 0.0};
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+        v[p] = load2<V2>(vq, i, n);
+        u[p] = load2<V2>(vq + n, i, n);
+      }
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        t.x += v[p].x * x[p].x + u[p].x * y[p].x + v[p].y * x[p].y + u[p].y * y[p].y;
+        t.y += v[p].x * y[p].x - u[p].x * x[p].x + v[p].y * y[p].y - u[p].y * x[p].y;
+      }
+      double2& a = dots[(q - c0) * KR_THREADS + tid];
+      a.x += t.x;
+      a.y += t.y;
+    }
+  }
+  __syncthreads();
+  for (int q = tid >> 5; q < c1 - c0; q += KR_THREADS / 32) {
+    double2 t{0.0, 0.0};
+    for (int l = tid & 31; l < KR_THREADS; l += 32) {
+      const double2 a = dots[q * KR_THREADS + l];
+      t.x += a.x;
+      t.y += a.y;
+    }
+    t.x = warp_sum(t.x);
+    t.y = warp_sum(t.y);
+    if ((tid & 31) == 0) {
+      partial[(int64_t)(2 * q) * gridDim.x + blockIdx.x] = t.x;
+      partial[(int64_t)(2 * q + 1) * gridDim.x + blockIdx.x] = t.y;
+    }
+  }
+  if (add_partials(partial, 2 * (c1 - c0), c.h + 2 * c0, count))
+    for (int r = tid; r < 2 * (c1 - c0); r += KR_THREADS) c.h[2 * c0 + r] *= c.scale[c0 + r / 2];
+}
+
+// U_{j+1} = w' - sum_{i <= j} h_i s_i U_i into (or, oi); then the step's
+// coefficients, which the host reads from `host` (pinned) after the stream
+// has come this far.
+template <bool V2, int P>
+__global__ void __launch_bounds__(KR_THREADS, 2)
+k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __restrict__ yr,
+                 const double* __restrict__ yi, int64_t n, int j, double* __restrict__ outr,
+                 double* __restrict__ outi, LanczosCoef c, double* __restrict__ partial,
+                 unsigned* __restrict__ count, double* __restrict__ host) {
+  __shared__ double2 hs[128];
+  __shared__ double red[KR_THREADS / 32];
+  const int tid = threadIdx.x;
+  for (int i = tid; i <= j; i += KR_THREADS)
+    hs[i] = double2{c.h[2 * i] * c.scale[i], c.h[2 * i + 1] * c.scale[i]};
+  const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
+  const double ar = c.a[0] * s, ai = c.a[1] * s;
+  __syncthreads();
+  const double* uj = U + (int64_t)j * ldv;
+  const double* up = j > 0 ? uj - ldv : uj;
+  double nrm = 0.0;
+  const int64_t tile = (int64_t)KR_THREADS * 2 * P;
+  for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
+    double2 x[P], y[P];
+    const int64_t i0 = base + (int64_t)tid * 2;
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+      x[p] = load2<V2>(yr, i, n);
+      y[p] = load2<V2>(yi, i, n);
+      const double2 v = load2<V2>(uj, i, n), u = load2<V2>(uj + n, i, n);
+      const double2 pr = load2<V2>(up, i, n), pi = load2<V2>(up + n, i, n);
+      local_step(x[p].x, y[p].x, s, b, pr.x, pi.x, ar, ai, v.x, u.x);
+      local_step(x[p].y, y[p].y, s, b, pr.y, pi.y, ar, ai, v.y, u.y);
+    }
+#pragma unroll 2
+    for (int q = 0; q <= j; ++q) {
+      const double* vq = U + (int64_t)q * ldv;
+      const double2 h = hs[q];
+      double2 v[P], u[P];
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+        v[p] = load2<V2>(vq, i, n);
+        u[p] = load2<V2>(vq + n, i, n);
+      }
+#pragma unroll
+      for (int p = 0; p < P; ++p) {
+        x[p].x -= h.x * v[p].x - h.y * u[p].x;
+        y[p].x -= h.x * u[p].x + h.y * v[p].x;
+        x[p].y -= h.x * v[p].y - h.y * u[p].y;
+        y[p].y -= h.x * u[p].y + h.y * v[p].y;
+      }
+    }
+#pragma unroll
+    for (int p = 0; p < P; ++p) {
+      const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
+      store2<V2>(outr, i, n, x[p]);
+      store2<V2>(outi, i, n, y[p]);
+      nrm += x[p].x * x[p].x + y[p].x * y[p].x + x[p].y * x[p].y + y[p].y * y[p].y;
+    }
+  }
+  nrm = warp_sum(nrm);
+  if ((tid & 31) == 0) red[tid >> 5] = nrm;
+  __syncthreads();
+  if (tid == 0) {
+    double t = 0.0;
+    for (int w = 0; w < KR_THREADS / 32; ++w) t += red[w];
+    partial[blockIdx.x] = t;
+  }
+  if (add_partials(partial, 1, c.nrm2, count) && tid == 0) {
+    const double a = c.a[0] + c.h[2 * j];
+    const double be = sqrt(fmax(0.0, *c.nrm2));
+    c.beta[j] = be;
+    // an exhausted Krylov space: the next basis vector counts as zero
+    c.scale[j + 1] = be > 1e-14 * fmax(1.0, fabs(a)) ? 1.0 / be : 0.0;
+    host[0] = a;
+    host[1] = be;
+    __threadfence_system();
+  }
 }
 
 // y = s * x with s read from the device; `inv_sqrt` takes s = 1 / sqrt(*p)
@@ -392,7 +592,7 @@ int launch_block_axpy(const AxpyBlock* d_blocks, int nblocks, const AxpyTerm* d_
 }
 
 // ---- Krylov helpers ---------------------------------------------------------
-int VecOps::init(int64_t n_) {
+int VecOps::init(int64_t n_, cudaStream_t st) {
   n = n_;
   nb = grid_for(n, RED_THREADS);
   if (nb > 1024) nb = 1024;
@@ -400,7 +600,8 @@ int VecOps::init(int64_t n_) {
   CMPS_CUDA(dmalloc(&d_coef, sizeof(double) * kCoefDoubles));
   CMPS_CUDA(dmalloc(&d_small, sizeof(double) * 2 * 128 * 2));
   CMPS_CUDA(dmalloc(&d_pidx, sizeof(int64_t) * nb));
-  return CMPS_OK;
+  CMPS_CUDA(dmalloc(&d_count, sizeof(unsigned)));
+  return zero_wait(d_count, sizeof(unsigned), st);
 }
 
 void VecOps::release() {
@@ -408,6 +609,8 @@ void VecOps::release() {
   if (d_small) dfree(d_small);
   if (d_pidx) dfree(d_pidx);
   if (d_coef) dfree(d_coef);
+  if (d_count) dfree(d_count);
+  d_count = nullptr;
   d_partial = d_small = d_coef = nullptr;
   d_pidx = nullptr;
 }
@@ -496,34 +699,9 @@ int VecOps::mdot_dev(const double* Vr, const double* Vi, int64_t ldv, int k, con
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (n + tile - 1) / tile));
   const int rows = 2 * k + 1;
   const size_t smem = sizeof(double) * (KR_THREADS / 32) * rows;
-  k_mdot<<<g, KR_THREADS, smem, st>>>(Vr, Vi, ldv, k, const_cast<double*>(wr), const_cast<double*>(wi), n, nullptr,
-                                      nullptr, nullptr, d_partial);
+  k_mdot<<<g, KR_THREADS, smem, st>>>(Vr, Vi, ldv, k, wr, wi, n, d_partial);
   CMPS_CUDA(cudaGetLastError());
   k_reduce_rows<<<rows, RED_THREADS, 0, st>>>(d_partial, g, rows, d_out);
-  CMPS_CUDA(cudaGetLastError());
-  return CMPS_OK;
-}
-
-int VecOps::update_mdot_dev(const double* d_c, const double* ur, const double* ui, const double* Vr, const double* Vi,
-                            int64_t ldv, int k, double* wr, double* wi, double* d_out, cudaStream_t st) {
-  if (k < 0 || k > 128) return fail(CMPS_ERR_ARG, "krylov dimension above 128");
-  const int64_t tile = (int64_t)KR_THREADS * KR_E;
-  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(nb, (n + tile - 1) / tile));
-  const int rows = 2 * k + 1;
-  const size_t smem = sizeof(double) * (KR_THREADS / 32) * rows;
-  k_mdot<<<g, KR_THREADS, smem, st>>>(Vr, Vi, ldv, k, wr, wi, n, d_c, ur, ui, d_partial);
-  CMPS_CUDA(cudaGetLastError());
-  k_reduce_rows<<<rows, RED_THREADS, 0, st>>>(d_partial, g, rows, d_out);
-  CMPS_CUDA(cudaGetLastError());
-  return CMPS_OK;
-}
-
-int VecOps::axpy_dot_dev(const double* pr, const double* pi, const double* d_beta, const double* vr, const double* vi,
-                         double* wr, double* wi, double* d_out, cudaStream_t st) {
-  const int g = std::min(nb, grid_for(n, KR_THREADS));
-  k_axpy_dot<<<g, KR_THREADS, 0, st>>>(pr, pi, d_beta, vr, vi, wr, wi, n, d_partial);
-  CMPS_CUDA(cudaGetLastError());
-  k_reduce_rows<<<2, RED_THREADS, 0, st>>>(d_partial, g, 2, d_out);
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }
@@ -539,11 +717,46 @@ int VecOps::maxpy_norm_dev(const double* Vr, const double* Vi, int64_t ldv, int 
   return CMPS_OK;
 }
 
-int VecOps::lanczos_coef(const double* d_a1, const double* d_a2, const double* d_nrm2, int j, double* d_alpha,
-                         double* d_beta, double* d_scale, cudaStream_t st) {
-  k_lanczos_coef<<<1, 32, 0, st>>>(d_a1, d_a2, d_nrm2, j, d_alpha, d_beta, d_scale);
+LanczosCoef VecOps::lanczos_coef() const {
+  double* p = d_coef;
+  return LanczosCoef{p, p + 8, p + 280, p + 408, p + 544};
+}
+
+// Tiles of 512 or 2048 elements: the small ones spread a short vector (the
+// XXZ chain's few thousand entries) over more CTAs; two CTAs per SM at most.
+template <bool V2, int P>
+static int lanczos_step(const VecOps& o, const double* U, int64_t ldv, const double* yr, const double* yi, int j,
+                        double* outr, double* outi, double* host, cudaStream_t st) {
+  const LanczosCoef c = o.lanczos_coef();
+  const int64_t tiles = (o.n + (int64_t)KR_THREADS * 2 * P - 1) / ((int64_t)KR_THREADS * 2 * P);
+  const int g = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(o.nb, 296), tiles));
+  const double* uj = U + (int64_t)j * ldv;
+  k_lanczos_dot<V2, P><<<g, KR_THREADS, 0, st>>>(uj, uj + o.n, yr, yi, o.n, j, c, o.d_partial, o.d_count);
+  CMPS_CUDA(cudaGetLastError());
+  constexpr int kChunk = 24;  // vectors per launch of the products: 96 KB of partial sums
+  CMPS_TRY(ensure_smem_optin((const void*)k_lanczos_mdot<V2, P>, kChunk * KR_THREADS * (int)sizeof(double2)));
+  for (int c0 = 0; c0 <= j; c0 += kChunk) {
+    const int c1 = std::min(j + 1, c0 + kChunk);
+    k_lanczos_mdot<V2, P><<<g, KR_THREADS, (size_t)(c1 - c0) * KR_THREADS * sizeof(double2), st>>>(
+        U, ldv, yr, yi, o.n, j, c0, c1, c, o.d_partial, o.d_count);
+    CMPS_CUDA(cudaGetLastError());
+  }
+  k_lanczos_update<V2, P><<<g, KR_THREADS, 0, st>>>(U, ldv, yr, yi, o.n, j, outr, outi, c, o.d_partial, o.d_count,
+                                                    host);
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
+}
+
+int VecOps::lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, int j, double* outr,
+                    double* outi, double* host, cudaStream_t st) {
+  if (j < 0 || j > 126) return fail(CMPS_ERR_ARG, "krylov dimension above 127");
+  const bool even = n % 2 == 0 && ldv % 2 == 0 &&
+                    (((uintptr_t)U | (uintptr_t)yr | (uintptr_t)yi | (uintptr_t)outr | (uintptr_t)outi) & 15) == 0;
+  const bool wide = n >= (int64_t)148 * 2 * 2048;
+  if (even && wide) return lanczos_step<true, 4>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
+  if (even) return lanczos_step<true, 1>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
+  if (wide) return lanczos_step<false, 4>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
+  return lanczos_step<false, 1>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
 }
 
 int VecOps::scale_dev(const double* xr, const double* xi, const double* d_s, bool inv_sqrt, double* yr, double* yi,

@@ -6,6 +6,13 @@
 
 namespace cmps {
 
+// Device-resident coefficients of a Lanczos cycle: the local projection a (2),
+// the Gram-Schmidt products h (2 per basis vector), beta_j and the scale s_j
+// of basis vector j (V_j = s_j U_j), and |U_{j+1}|^2.
+struct LanczosCoef {
+  double *a, *h, *beta, *scale, *nrm2;
+};
+
 // Planar FP64 complex vectors of a fixed length n; reductions are two-pass
 // (per-CTA partials, then a fixed-order reduction) so results are
 // deterministic run to run.
@@ -15,7 +22,7 @@ struct VecOps {
   double* d_partial = nullptr;
   double* d_small = nullptr;
   int64_t* d_pidx = nullptr;
-  int init(int64_t n);
+  int init(int64_t n, cudaStream_t st);
   void release();
   // h[j] = <V_j, w> (conjugate-linear in V), k vectors with stride ldv; h_host gets 2k doubles.
   int multidot(const double* Vr, const double* Vi, int64_t ldv, int k, const double* wr, const double* wi,
@@ -40,16 +47,15 @@ struct VecOps {
   // w -= sum_j h_j V_j with h = d_h (2k doubles); *d_nrm2 = |w|^2 afterwards.
   int maxpy_norm_dev(const double* Vr, const double* Vi, int64_t ldv, int k, const double* d_h, double* wr,
                      double* wi, double* d_nrm2, cudaStream_t st);
-  // w -= c u (c = d_c[0] + i d_c[1]), then as mdot_dev with the updated w.
-  int update_mdot_dev(const double* d_c, const double* ur, const double* ui, const double* Vr, const double* Vi,
-                      int64_t ldv, int k, double* wr, double* wi, double* d_out, cudaStream_t st);
-  // w -= (*d_beta) p (skipped when pr is null), then d_out[0..1] = <v, w>.
-  int axpy_dot_dev(const double* pr, const double* pi, const double* d_beta, const double* vr, const double* vi,
-                   double* wr, double* wi, double* d_out, cudaStream_t st);
-  // alpha_j = *d_a1 + *d_a2, beta_j = sqrt(*d_nrm2), and the scale of the next
-  // basis vector (0 when the Krylov space is exhausted).
-  int lanczos_coef(const double* d_a1, const double* d_a2, const double* d_nrm2, int j, double* d_alpha,
-                   double* d_beta, double* d_scale, cudaStream_t st);
+  // Step j of a Lanczos cycle with full re-orthogonalisation (kernels.cu):
+  // basis vectors U_0 .. U_j at U + i ldv (real plane, imaginary plane n
+  // further), y = H U_j; the next vector into (outr, outi), alpha_j and beta_j
+  // into host[0..1] (pinned memory) once the stream has come this far.  The
+  // cycle's first scale, lanczos_coef().scale[0], is the caller's.
+  int lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, int j, double* outr, double* outi,
+              double* host, cudaStream_t st);
+  LanczosCoef lanczos_coef() const;
+  unsigned* d_count = nullptr;  // CTAs of the current launch that have finished
   // y = s x with s = *d_s, or s = 1 / sqrt(*d_s) when inv_sqrt.
   int scale_dev(const double* xr, const double* xi, const double* d_s, bool inv_sqrt, double* yr, double* yi,
                 cudaStream_t st);

@@ -441,43 +441,67 @@ static double launch_cost(const GemmPlan& p) {
 }
 static int pick_shape64(const GemmPlan& p) { return launch_cost<TileQ>(p) <= 1.1 * launch_cost<TileS>(p) ? 0 : 1; }
 
-// The tiles of the plan's tasks.  Tasks with long K come first (in octaves of
-// K, so that tasks sharing operands stay neighbours): the launch's last wave
-// is then made of short tiles.
+// One block per listed task writes the task's tiles, rows of tiles first: a
+// plan has a few thousand tasks and up to some 10^5 tiles.
+struct TaskTiles {
+  int32_t task, pm, pn, pad;
+  int64_t first;
+};
 template <class T>
-static void make_tiles(const GemmPlan& p, std::vector<GemmTile>& out) {
-  std::vector<std::pair<int, int32_t>> order;
+__global__ void k_expand_tiles(const TaskTiles* __restrict__ list, const GemmTask* __restrict__ tasks,
+                               GemmTile* __restrict__ tiles) {
+  const TaskTiles tt = list[blockIdx.x];
+  const GemmTask t = tasks[tt.task];
+  // slice counts differ by at most one over a task's tiles
+  const int64_t sM = (t.m + 7) / 8, sN = (t.n + 7) / 8;
+  for (int64_t i = threadIdx.x; i < (int64_t)tt.pm * tt.pn; i += blockDim.x) {
+    const int64_t a = i / tt.pn, b = i - a * tt.pn;
+    const int64_t ma = sM * a / tt.pm, nb = sN * b / tt.pn;
+    const int sm = (int)(sM * (a + 1) / tt.pm - ma), sn = (int)(sN * (b + 1) / tt.pn - nb);
+    int hm, hn, wml;
+    arrange<T>(sm, sn, hm, hn, wml);
+    tiles[tt.first + i] = GemmTile{tt.task, (int32_t)(8 * ma), (int32_t)(8 * nb),
+                                   sm | sn << 6 | wml << 12 | hm << 14 | hn << 20};
+  }
+}
+
+// The tiles of the plan's tasks, written on the device.  Tasks with long K
+// come first (in octaves of K, so that tasks sharing operands stay
+// neighbours): the launch's last wave is then made of short tiles.
+template <class T>
+static int make_tiles(const GemmPlan& p, GemmTiles& to, cudaStream_t st) {
+  std::vector<std::pair<int, TaskTiles>> order;
   int64_t total = 0;
   for (size_t i = 0; i < p.tasks.size(); ++i) {
     const GemmTask& t = p.tasks[i];
     if (t.m <= 0 || t.n <= 0) continue;
-    total += (int64_t)parts(t.m, T::BM / 8) * parts(t.n, T::BN / 8);
     int64_t k = 1;
     for (int q = t.t0; q < t.t1; ++q) k += (p.terms[q].k + BK - 1) / BK;
     int oct = 0;
     while (k >>= 1) ++oct;
-    order.push_back({-oct, (int32_t)i});
+    order.push_back({-oct, TaskTiles{(int32_t)i, parts(t.m, T::BM / 8), parts(t.n, T::BN / 8), 0, 0}});
   }
   std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first < b.first; });
-  out.reserve((size_t)total);
+  std::vector<TaskTiles> list;
+  list.reserve(order.size());
   for (auto& o : order) {
-    const GemmTask& t = p.tasks[o.second];
-    // slice counts differ by at most one over a task's tiles
-    const int pm = parts(t.m, T::BM / 8), pn = parts(t.n, T::BN / 8);
-    const int64_t sM = (t.m + 7) / 8, sN = (t.n + 7) / 8;
-    for (int a = 0; a < pm; ++a) {
-      const int64_t ma = sM * a / pm;
-      const int sm = (int)(sM * (a + 1) / pm - ma);
-      for (int b = 0; b < pn; ++b) {
-        const int64_t nb = sN * b / pn;
-        const int sn = (int)(sN * (b + 1) / pn - nb);
-        int hm, hn, wml;
-        arrange<T>(sm, sn, hm, hn, wml);
-        out.push_back(GemmTile{o.second, (int32_t)(8 * ma), (int32_t)(8 * nb),
-                               sm | sn << 6 | wml << 12 | hm << 14 | hn << 20});
-      }
-    }
+    o.second.first = total;
+    total += (int64_t)o.second.pm * o.second.pn;
+    list.push_back(o.second);
   }
+  to.n = total;
+  if (!total) return CMPS_OK;
+  TaskTiles* d_list = nullptr;
+  CMPS_CUDA(dmalloc((void**)&to.d, (size_t)total * sizeof(GemmTile)));
+  CMPS_CUDA(dmalloc((void**)&d_list, list.size() * sizeof(TaskTiles)));
+  int rc = copy_wait(d_list, list.data(), list.size() * sizeof(TaskTiles), cudaMemcpyHostToDevice, st);
+  if (rc == CMPS_OK) {
+    k_expand_tiles<T><<<(unsigned)list.size(), 128, 0, st>>>(d_list, p.d_tasks, to.d);
+    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
+      rc = fail(CMPS_ERR_CUDA, "GEMM plan: tile list");
+  }
+  dfree(d_list);
+  return rc;
 }
 
 // Tile shape of a plan in FP32 (cgemm_fp32.cu, whole tiles): the shape whose
@@ -508,30 +532,30 @@ static int pick_shape32(const GemmPlan& p) {
 int GemmPlan::retile(bool fp32, int s, cudaStream_t st) {
   if (s < 0 || s >= (fp32 ? 3 : kNumShapes64)) return fail(CMPS_ERR_ARG, "GEMM plan: unknown tile shape");
   if (!d_tasks && !tasks.empty()) return fail(CMPS_ERR_STATE, "GEMM plan not uploaded");
-  std::vector<GemmTile> nt;
+  GemmTiles nt;
+  nt.shape = s;
+  int rc = CMPS_OK;
   if (!fp32) {
-    if (s == 0) make_tiles<TileQ>(*this, nt);
-    else make_tiles<TileS>(*this, nt);
+    rc = s == 0 ? make_tiles<TileQ>(*this, nt, st) : make_tiles<TileS>(*this, nt, st);
   } else {
     const int bm = kShapes32[s][0], bn = kShapes32[s][1];
+    std::vector<GemmTile> v;
     for (size_t i = 0; i < tasks.size(); ++i)
       for (int m0 = 0; m0 < tasks[i].m; m0 += bm)
-        for (int n0 = 0; n0 < tasks[i].n; n0 += bn) nt.push_back(GemmTile{(int32_t)i, m0, n0, 0});
-  }
-  GemmTile* d = nullptr;
-  if (!nt.empty()) {
-    CMPS_CUDA(dmalloc((void**)&d, nt.size() * sizeof(GemmTile)));
-    const int rc = copy_wait(d, nt.data(), nt.size() * sizeof(GemmTile), cudaMemcpyHostToDevice, st);
-    if (rc != CMPS_OK) {
-      dfree(d);
-      return rc;
+        for (int n0 = 0; n0 < tasks[i].n; n0 += bn) v.push_back(GemmTile{(int32_t)i, m0, n0, 0});
+    nt.n = (int64_t)v.size();
+    if (nt.n) {
+      CMPS_CUDA(dmalloc((void**)&nt.d, v.size() * sizeof(GemmTile)));
+      rc = copy_wait(nt.d, v.data(), v.size() * sizeof(GemmTile), cudaMemcpyHostToDevice, st);
     }
+  }
+  if (rc != CMPS_OK) {
+    if (nt.d) dfree(nt.d);
+    return rc;
   }
   GemmTiles& to = fp32 ? t32 : t64;
   if (to.d) dfree(to.d);
-  to.d = d;
-  to.n = (int64_t)nt.size();
-  to.shape = s;
+  to = nt;
   return CMPS_OK;
 }
 
@@ -580,7 +604,6 @@ int autotune_plan(GemmPlan& p, int role, bool fp32, const std::function<int()>& 
     }
     float ms = 0.0f;
     cudaEventElapsedTime(&ms, e0, e1);
-    if (std::getenv("CMPS_TUNE_TRACE")) std::fprintf(stderr, "  role %d shape %d: %.4f ms\n", role, s, ms / 3);
     if (s == heuristic) heur = ms;
     if (s == 0 || ms < best) {
       best = ms;

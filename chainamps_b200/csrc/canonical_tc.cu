@@ -679,7 +679,7 @@ int build_canonical_tc(Heff& H) {
         }
     }
     if (out) tc::mark_vector_stores(p, out, out_len);  // mode 3: BF16 output in 16-byte stores
-    return tc::finish_plan(p, true, true, brows, !grouped, true);
+    return tc::finish_plan(p, true, true, brows, grouped ? tc::kAsListed : tc::kHeaviestFirst, true);
   };
   CMPS_TRY(build_plan(T->pR, fR, true, T->zv, T->zv_len));
   CMPS_TRY(build_plan(T->pW2, fW2, true, T->y, T->y_len));

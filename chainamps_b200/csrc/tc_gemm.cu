@@ -821,15 +821,19 @@ tc_split_gemm(const TcTile* __restrict__ tiles, int ntiles, const TcTask* __rest
 
 int smem_bytes() { return kSmemBytes; }
 
+int num_sms() {
+  int dev = 0, sms = 148;
+  cudaGetDevice(&dev);
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  return std::max(sms, 1);
+}
+
 int launch(int mode, const TcPlan& p, float* out32, int64_t out32_plane, double* out64, int64_t out64_plane,
            const float* ain, int64_t a_plane, int* d_err, cudaStream_t st) {
   if (p.tiles.empty()) return CMPS_OK;
   if (p.tiles.size() > 0x7fffffffull) return fail(CMPS_ERR_ARG, "too many tcgen05 tiles");
-  int dev = 0, sms = 148;
-  cudaGetDevice(&dev);
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
   const int ntiles = (int)p.tiles.size();
-  const unsigned grid = (unsigned)std::min(ntiles, sms);
+  const unsigned grid = (unsigned)std::min(ntiles, num_sms());
   if (mode == 1 || mode == 3 || mode == 4) {
     if (!p.d_amaps) return fail(CMPS_ERR_STATE, "tcgen05: no A tensor maps");
     auto kern = mode == 1 ? tc_split_gemm<1> : mode == 3 ? tc_split_gemm<3> : tc_split_gemm<4>;

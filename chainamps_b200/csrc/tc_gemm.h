@@ -74,6 +74,8 @@ struct TcPlan {
 };
 
 int smem_bytes();
+// SMs of the current device: the CTAs of a launch, one persistent CTA each.
+int num_sms();
 // 3-D tensor map (K, rows, 4 planes) over one operand block of FP32 or BF16
 // elements at `base` (plane 0), planes `plane` elements apart, rows `ld`
 // elements apart; the block must fit in `room` elements from base.  Box: 64
@@ -84,12 +86,14 @@ int encode_map(bool bf16, const void* base, int64_t K, int64_t rows, int64_t ld,
 void add_tiles(TcPlan& p, int32_t task, int32_t m, int32_t n);
 // The same over the row ranges `used` (begin, end; ascending) only.
 void add_tiles(TcPlan& p, int32_t task, const std::vector<std::pair<int32_t, int32_t>>& used, int32_t n);
-// Completes a plan built term by term: k-steps per tile, optionally the
-// heaviest tiles first, and checks every term, task, segment list and tile.
+// The order in which a plan's tiles are dealt to the SMs.
+enum TileOrder { kAsListed, kHeaviestFirst, kHeaviestInTurns };
+// Completes a plan built term by term: k-steps per tile, the tiles' order, and
+// checks every term, task, segment list and tile.
 // by_tma: the A operands are tensor maps (else converter descriptors);
 // b_rows: the row count each B map was encoded with; wide_ok: narrow BF16
 // tiles take the four-plane MMA form.
-int finish_plan(TcPlan& p, bool bf16, bool by_tma, const std::vector<int32_t>& b_rows, bool heaviest_first,
+int finish_plan(TcPlan& p, bool bf16, bool by_tma, const std::vector<int32_t>& b_rows, TileOrder order,
                 bool wide_ok = false);
 // Mode 3: marks the tasks whose output takes 16-byte stores of 8-row runs
 // (rows contiguous, M a multiple of 8, segment starts and column / plane

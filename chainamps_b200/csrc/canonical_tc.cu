@@ -67,24 +67,58 @@ struct XinBlock {
   int32_t n1p, n2p, d2p, pad;
 };
 
-// theta (FP64 planes) -> Theta_in (four BF16 planes): one warp per run of d2
-// consecutive elements, which are consecutive in both layouts.
+// theta (FP64 planes) -> Theta_in (four BF16 planes): one warp per (i, a0), whose
+// n2 d2 elements are consecutive in theta, and in Theta_in too where d2 needs
+// no padding.  Two elements per lane (16-byte loads) where theta's offsets are
+// even throughout; four such pairs in flight.
+template <bool V2>
+__device__ __forceinline__ void gather_row(const double* __restrict__ re, const double* __restrict__ im,
+                                           uint16_t* __restrict__ o, int64_t plane, int n, int d2, int d2p) {
+  const int lane = threadIdx.x & 31;
+  constexpr int W = V2 ? 2 : 1;
+  for (int e0 = lane * W; e0 < n; e0 += 4 * 32 * W) {
+    double xr[4][W], xi[4][W];
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = e0 + q * 32 * W;
+      if (e >= n) continue;
+      if (V2) {
+        const double2 a = *reinterpret_cast<const double2*>(re + e), b = *reinterpret_cast<const double2*>(im + e);
+        xr[q][0] = a.x, xr[q][W - 1] = a.y, xi[q][0] = b.x, xi[q][W - 1] = b.y;
+      } else {
+        xr[q][0] = re[e];
+        xi[q][0] = im[e];
+      }
+    }
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = e0 + q * 32 * W;
+      if (e >= n) continue;
+      const int at = d2 == d2p ? e : e / d2 * d2p + e % d2;
+      uint16_t p[4][W];
+#pragma unroll
+      for (int w = 0; w < W; ++w) split4(xr[q][w], xi[q][w], &p[0][w], &p[1][w], &p[2][w], &p[3][w]);
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        if (V2) *reinterpret_cast<uint32_t*>(o + at + k * plane) = (uint32_t)p[k][0] | (uint32_t)p[k][W - 1] << 16;
+        else o[at + k * plane] = p[k][0];
+      }
+    }
+  }
+}
+
 __global__ void __launch_bounds__(256) k_gather_theta(const XinBlock* __restrict__ blocks,
                                                       const double* __restrict__ re, const double* __restrict__ im,
                                                       uint16_t* __restrict__ dst, int64_t plane) {
   const XinBlock b = blocks[blockIdx.y];
-  const int64_t runs = (int64_t)b.d0 * b.n1 * b.n2;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t step = (int64_t)gridDim.x * (blockDim.x >> 5);
-  for (int64_t r = (int64_t)blockIdx.x * (blockDim.x >> 5) + warp; r < runs; r += step) {
-    const int64_t j = r % b.n2, t = r / b.n2;
-    const int64_t i = t % b.n1, a0 = t / b.n1;
-    const int64_t s = b.src + (i * b.d0 + a0) * b.ncols + j * b.d2;
-    const int64_t d = b.dst + ((a0 * b.n1p + i) * b.n2p + j) * b.d2p;
-    for (int a2 = lane; a2 < b.d2; a2 += 32) {
-      uint16_t* o = dst + d + a2;
-      split4(re[s + a2], im[s + a2], o, o + plane, o + 2 * plane, o + 3 * plane);
-    }
+  const int rows = b.d0 * b.n1;
+  const bool even = ((b.src | b.ncols | b.d2) & 1) == 0 && (((uintptr_t)re | (uintptr_t)im) & 15) == 0;
+  for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += gridDim.x * (blockDim.x >> 5)) {
+    const int a0 = r / b.n1, i = r - a0 * b.n1;
+    const int64_t s = b.src + ((int64_t)i * b.d0 + a0) * b.ncols;
+    uint16_t* o = dst + b.dst + ((int64_t)a0 * b.n1p + i) * b.n2p * b.d2p;
+    if (even) gather_row<true>(re + s, im + s, o, plane, b.n2 * b.d2, b.d2, b.d2p);
+    else gather_row<false>(re + s, im + s, o, plane, b.n2 * b.d2, b.d2, b.d2p);
   }
 }
 
@@ -259,7 +293,9 @@ int build_canonical_tc(Heff& H) {
     b.dst = T->xin_len;
     xoff[{m, c1, c2}] = T->xin_len;
     T->xin_len += align64(pad8(b.d0) * b.n1p * b.n2p * b.d2p);
-    T->max_runs = std::max<int64_t>(T->max_runs, (int64_t)b.d0 * b.n1 * b.n2);
+    if ((int64_t)b.d0 * b.n1 > 0x7fffffff || (int64_t)b.n2 * b.d2 > 0x3fffffff)
+      return fail(CMPS_ERR_ARG, "canonical tcgen05 form: theta block too large");
+    T->max_runs = std::max<int64_t>(T->max_runs, (int64_t)b.d0 * b.n1);
     xb.push_back(b);
   }
   if (xb.size() > 65535) return fail(CMPS_ERR_ARG, "canonical tcgen05 form: too many theta blocks");

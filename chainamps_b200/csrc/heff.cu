@@ -376,53 +376,58 @@ int Heff::allowed_indices(int64_t* host_out) const {
 // ARPACK order -> sector blocks: CTA = (group of <= 32 columns, 32 rows).
 // Reads run down each ARPACK column (contiguous), writes along theta rows
 // (the group's columns are consecutive theta columns).
+// HBM bound (16 bytes in, 16 out per entry).  Two dependent reads of
+// descriptors stand before the data (four before: gather 0.27 ms at 33.5M
+// entries, now 0.205).  The gather takes the tile's 64 rows in one CTA, so that
+// more reads are in flight; the scatter gives each half of them a CTA of its own
+// (64 rows there: 0.30 against 0.257 ms).
 template <bool PACK>
 __global__ void __launch_bounds__(256) k_pack_tiles(const Heff::PackTile* __restrict__ tiles,
                                                     const Heff::PackGroup* __restrict__ groups,
-                                                    const int32_t* __restrict__ gcols,
-                                                    const Heff::MapCol* __restrict__ cols,
-                                                    const Heff::MapSec* __restrict__ secs,
+                                                    const int64_t* __restrict__ starts,
                                                     const int64_t* __restrict__ rowth, double2* __restrict__ arp,
                                                     double* __restrict__ re, double* __restrict__ im) {
-  __shared__ double2 t[32][33];  // [column j][row r]
-  const Heff::PackTile tl = tiles[blockIdx.x];
+  constexpr int ROWS = PACK ? 64 : 32, LD = ROWS + 1, E = ROWS / 8;  // E elements per thread
+  __shared__ double2 t[32 * LD];  // [column j][row r]
+  const Heff::PackTile tl = tiles[PACK ? blockIdx.x : blockIdx.x >> 1];
   const Heff::PackGroup g = groups[tl.group];
-  const Heff::MapSec s = secs[g.m];
+  const int64_t r0 = tl.r0 + (PACK ? 0 : 32 * (int)(blockIdx.x & 1));
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
-  const int64_t left = s.nrows - tl.r0;
-  const int nr = left < 32 ? (int)left : 32;
+  const int nr = (int)min((int64_t)ROWS, g.nrows - r0), nc = (int)g.cnt;
+  if (nr <= 0) return;
+  const int64_t* rows = rowth + g.rowstart + r0;
+  const int64_t* col = starts + g.off;
+  // along an ARPACK column: column j, row r of element k; along a theta row: row ty + 8 k, column tx
+  auto j_of = [&](int k) { return ty + 8 * (k / (ROWS / 32)); };
+  auto r_of = [&](int k) { return tx + 32 * (k % (ROWS / 32)); };
   if (PACK) {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int j = ty + 8 * k, r = tx;
-      if (j < g.cnt && r < nr) t[j][r] = arp[cols[gcols[g.off + j]].start + tl.r0 + r];
-    }
+    for (int k = 0; k < E; ++k)
+      if (j_of(k) < nc && r_of(k) < nr) t[j_of(k) * LD + r_of(k)] = arp[col[j_of(k)] + r0 + r_of(k)];
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int r = ty + 8 * k, j = tx;
-      if (j < g.cnt && r < nr) {
-        const int64_t p = s.base + rowth[s.rowstart + tl.r0 + r] * s.ncols + cols[gcols[g.off + j]].colth;
-        const double2 v = t[j][r];
-        re[p] = v.x;
-        im[p] = v.y;
+    for (int k = 0; k < E; ++k) {
+      const int r = ty + 8 * k;
+      if (tx < nc && r < nr) {
+        const int64_t p = g.base + rows[r] * g.ncols + tx;
+        const double2 w = t[tx * LD + r];
+        re[p] = w.x;
+        im[p] = w.y;
       }
     }
   } else {
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int r = ty + 8 * k, j = tx;
-      if (j < g.cnt && r < nr) {
-        const int64_t p = s.base + rowth[s.rowstart + tl.r0 + r] * s.ncols + cols[gcols[g.off + j]].colth;
-        t[j][r] = make_double2(re[p], im[p]);
+    for (int k = 0; k < E; ++k) {
+      const int r = ty + 8 * k;
+      if (tx < nc && r < nr) {
+        const int64_t p = g.base + rows[r] * g.ncols + tx;
+        t[tx * LD + r] = make_double2(re[p], im[p]);
       }
     }
     __syncthreads();
 #pragma unroll
-    for (int k = 0; k < 4; ++k) {
-      const int j = ty + 8 * k, r = tx;
-      if (j < g.cnt && r < nr) arp[cols[gcols[g.off + j]].start + tl.r0 + r] = t[j][r];
-    }
+    for (int k = 0; k < E; ++k)
+      if (j_of(k) < nc && r_of(k) < nr) arp[col[j_of(k)] + r0 + r_of(k)] = t[j_of(k) * LD + r_of(k)];
   }
 }
 
@@ -436,7 +441,7 @@ int Heff::build_pack(cudaStream_t st) {
   }
   std::vector<std::vector<int64_t>> elems(A2.nsec());
   for (int64_t a2 = 0; a2 < A2.size(); ++a2) elems[A2.esec[a2]].push_back(a2);
-  std::vector<int32_t> gcols;
+  std::vector<int64_t> starts;
   std::vector<PackGroup> groups;
   std::vector<PackTile> tiles;
   for (int m = 0; m < (int)th.mq.size(); ++m)
@@ -445,40 +450,34 @@ int Heff::build_pack(cudaStream_t st) {
       const int t = A2.find(rules.add(th.mq[m], sigq[s2]));
       const std::vector<int64_t>& el = elems[t];
       for (size_t e0 = 0; e0 < el.size(); e0 += 32) {
-        PackGroup g{(int64_t)gcols.size(), (int32_t)std::min<size_t>(32, el.size() - e0), m};
+        PackGroup g{(int64_t)starts.size(), th.base[m] + th.coloff[m][s2] + (int64_t)e0, th.ncols[m],
+                    map_secs[m].rowstart,   th.nrows[m], (int64_t)std::min<size_t>(32, el.size() - e0)};
         for (int j = 0; j < g.cnt; ++j) {
           const int32_t c = col_of[(size_t)el[e0 + j] * d + s2];
           if (c < 0 || map_cols[c].m != m || map_cols[c].colth != th.coloff[m][s2] + (int64_t)(e0 + j))
             return fail(CMPS_ERR_STATE, "internal: pack group columns not consecutive");
-          gcols.push_back(c);
+          starts.push_back(map_cols[c].start);
         }
-        for (int64_t r0 = 0; r0 < th.nrows[m]; r0 += 32) tiles.push_back(PackTile{(int32_t)groups.size(), (int32_t)r0});
+        for (int64_t r0 = 0; r0 < th.nrows[m]; r0 += 64) tiles.push_back(PackTile{(int32_t)groups.size(), (int32_t)r0});
         groups.push_back(g);
       }
     }
-  if (tiles.size() > 0x7fffffffull) return fail(CMPS_ERR_ARG, "too many pack tiles");
+  if (tiles.size() > 0x3fffffffull) return fail(CMPS_ERR_ARG, "too many pack tiles");
   n_pack_tiles = 0;
   if (tiles.empty()) return CMPS_OK;
   auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
-  const size_t b_cols = al(sizeof(MapCol) * map_cols.size()), b_secs = al(sizeof(MapSec) * map_secs.size()),
-               b_rowth = al(sizeof(int64_t) * map_rowth.size()), b_gcols = al(sizeof(int32_t) * gcols.size()),
+  const size_t b_rowth = al(sizeof(int64_t) * map_rowth.size()), b_starts = al(sizeof(int64_t) * starts.size()),
                b_groups = al(sizeof(PackGroup) * groups.size()), b_tiles = al(sizeof(PackTile) * tiles.size());
   if (d_pack) dfree(d_pack);
   d_pack = nullptr;
-  CMPS_CUDA(dmalloc(&d_pack, b_cols + b_secs + b_rowth + b_gcols + b_groups + b_tiles));
+  CMPS_CUDA(dmalloc(&d_pack, b_rowth + b_starts + b_groups + b_tiles));
   char* p = (char*)d_pack;
-  d_map_cols = (const MapCol*)p;
-  CMPS_TRY(copy_wait(p, map_cols.data(), sizeof(MapCol) * map_cols.size(), cudaMemcpyHostToDevice, st));
-  p += b_cols;
-  d_map_secs = (const MapSec*)p;
-  CMPS_TRY(copy_wait(p, map_secs.data(), sizeof(MapSec) * map_secs.size(), cudaMemcpyHostToDevice, st));
-  p += b_secs;
   d_map_rowth = (const int64_t*)p;
   CMPS_TRY(copy_wait(p, map_rowth.data(), sizeof(int64_t) * map_rowth.size(), cudaMemcpyHostToDevice, st));
   p += b_rowth;
-  d_pack_gcols = (const int32_t*)p;
-  CMPS_TRY(copy_wait(p, gcols.data(), sizeof(int32_t) * gcols.size(), cudaMemcpyHostToDevice, st));
-  p += b_gcols;
+  d_pack_starts = (const int64_t*)p;
+  CMPS_TRY(copy_wait(p, starts.data(), sizeof(int64_t) * starts.size(), cudaMemcpyHostToDevice, st));
+  p += b_starts;
   d_pack_groups = (const PackGroup*)p;
   CMPS_TRY(copy_wait(p, groups.data(), sizeof(PackGroup) * groups.size(), cudaMemcpyHostToDevice, st));
   p += b_groups;
@@ -490,16 +489,16 @@ int Heff::build_pack(cudaStream_t st) {
 
 int Heff::pack(const double* in, const Planar& out, cudaStream_t st) const {
   if (n_pack_tiles == 0) return CMPS_OK;
-  k_pack_tiles<true><<<(unsigned)n_pack_tiles, 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_gcols, d_map_cols,
-                                                             d_map_secs, d_map_rowth, (double2*)in, out.re(), out.im());
+  k_pack_tiles<true><<<(unsigned)n_pack_tiles, 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_starts, d_map_rowth,
+                                                             (double2*)in, out.re(), out.im());
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }
 
 int Heff::unpack(const Planar& in, double* out, cudaStream_t st) const {
   if (n_pack_tiles == 0) return CMPS_OK;
-  k_pack_tiles<false><<<(unsigned)n_pack_tiles, 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_gcols, d_map_cols,
-                                                              d_map_secs, d_map_rowth, (double2*)out, in.re(), in.im());
+  k_pack_tiles<false><<<(unsigned)(2 * n_pack_tiles), 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_starts,
+                                                                    d_map_rowth, (double2*)out, in.re(), in.im());
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }

@@ -76,21 +76,21 @@ struct Heff {
   // mode 0: ARPACK index -> theta offset; mode 1: -> full linear index
   int arpack_map(int mode, int64_t* d_out, cudaStream_t st) const;
   int allowed_indices(int64_t* host_out) const;
-  // ARPACK order <-> sector blocks as 32 x 32 transpose tiles: a group is up
-  // to 32 ARPACK columns of one (block m, sigma2) with consecutive a2
-  // positions, i.e. consecutive theta columns.
+  // ARPACK order <-> sector blocks as transpose tiles of 32 columns x 64 rows:
+  // a group is up to 32 ARPACK columns of one (block m, sigma2) with
+  // consecutive a2 positions, i.e. consecutive theta columns.
   struct PackGroup {
-    int64_t off;  // into the group column list
-    int32_t cnt, m;
+    int64_t off;               // into the group column starts (first ARPACK index of each column)
+    int64_t base, ncols;       // theta: first column of the group in row 0 of its block, row length
+    int64_t rowstart, nrows;   // rows of the block in ARPACK row order
+    int64_t cnt;               // columns
   };
   struct PackTile {
     int32_t group, r0;
   };
-  void* d_pack = nullptr;        // one allocation: cols, secs, rowth, group columns, groups, tiles
-  const MapCol* d_map_cols = nullptr;
-  const MapSec* d_map_secs = nullptr;
+  void* d_pack = nullptr;        // one allocation: rowth, group column starts, groups, tiles
   const int64_t* d_map_rowth = nullptr;
-  const int32_t* d_pack_gcols = nullptr;
+  const int64_t* d_pack_starts = nullptr;
   const PackGroup* d_pack_groups = nullptr;
   const PackTile* d_pack_tiles = nullptr;
   int64_t n_pack_tiles = 0;

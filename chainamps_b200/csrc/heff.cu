@@ -394,9 +394,13 @@ __global__ void __launch_bounds__(256) k_pack_tiles(const Heff::PackTile* __rest
   const int64_t r0 = tl.r0 + (PACK ? 0 : 32 * (int)(blockIdx.x & 1));
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
   const int nr = (int)min((int64_t)ROWS, g.nrows - r0), nc = (int)g.cnt;
-  if (nr <= 0) return;
+  if (nr <= 0) {
+    grid_wait();
+    return;
+  }
   const int64_t* rows = rowth + g.rowstart + r0;
   const int64_t* col = starts + g.off;
+  grid_wait();  // up to here only descriptors were read
   // along an ARPACK column: column j, row r of element k; along a theta row: row ty + 8 k, column tx
   auto j_of = [&](int k) { return ty + 8 * (k / (ROWS / 32)); };
   auto r_of = [&](int k) { return tx + 32 * (k % (ROWS / 32)); };
@@ -489,17 +493,15 @@ int Heff::build_pack(cudaStream_t st) {
 
 int Heff::pack(const double* in, const Planar& out, cudaStream_t st) const {
   if (n_pack_tiles == 0) return CMPS_OK;
-  k_pack_tiles<true><<<(unsigned)n_pack_tiles, 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_starts, d_map_rowth,
-                                                             (double2*)in, out.re(), out.im());
-  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(launch_chained(k_pack_tiles<true>, dim3((unsigned)n_pack_tiles), dim3(256), 0, st, d_pack_tiles,
+                           d_pack_groups, d_pack_starts, d_map_rowth, (double2*)in, out.re(), out.im()));
   return CMPS_OK;
 }
 
 int Heff::unpack(const Planar& in, double* out, cudaStream_t st) const {
   if (n_pack_tiles == 0) return CMPS_OK;
-  k_pack_tiles<false><<<(unsigned)(2 * n_pack_tiles), 256, 0, st>>>(d_pack_tiles, d_pack_groups, d_pack_starts,
-                                                                    d_map_rowth, (double2*)out, in.re(), in.im());
-  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(launch_chained(k_pack_tiles<false>, dim3((unsigned)(2 * n_pack_tiles)), dim3(256), 0, st, d_pack_tiles,
+                           d_pack_groups, d_pack_starts, d_map_rowth, (double2*)out, in.re(), in.im()));
   return CMPS_OK;
 }
 

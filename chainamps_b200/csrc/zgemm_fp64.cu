@@ -291,6 +291,7 @@ zgemm_grouped_fp64(const GemmTile* __restrict__ tiles, const GemmTask* __restric
     cp_commit();
     return kl;
   };
+  grid_wait();  // up to here only the plan was read
   int len0 = issue(0), len1 = issue(1);
   int buf = 0, since = 0;
   while (len0 > 0) {
@@ -356,9 +357,9 @@ int launch_variant(const GemmPlan& p, const Planar& A, const Planar& B, Planar& 
   CMPS_TRY(ensure_smem_optin((const void*)zgemm_grouped_fp64<T, AH, BH, NSPLIT, AREAL>, (int)T::SMEM_BYTES));
   if (p.t64.n <= 0) return CMPS_OK;
   if (p.t64.n > 0x7fffffff) return fail(CMPS_ERR_ARG, "too many GEMM tiles");
-  zgemm_grouped_fp64<T, AH, BH, NSPLIT, AREAL><<<(unsigned)p.t64.n, NTHREADS, T::SMEM_BYTES, st>>>(
-      p.t64.d, p.d_tasks, p.d_terms, A.re(), A.im() - A.re(), B.re(), B.im() - B.re(), C.re(), C.im() - C.re());
-  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(launch_chained(zgemm_grouped_fp64<T, AH, BH, NSPLIT, AREAL>, dim3((unsigned)p.t64.n), dim3(NTHREADS),
+                           T::SMEM_BYTES, st, p.t64.d, p.d_tasks, p.d_terms, A.re(), A.im() - A.re(), B.re(),
+                           B.im() - B.re(), C.re(), C.im() - C.re()));
   return CMPS_OK;
 }
 

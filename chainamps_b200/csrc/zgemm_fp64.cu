@@ -190,7 +190,10 @@ struct Acc {
 };
 
 // One stage of kl values of K for a warp's NI x NJ slices, straight-line.
-template <class T, bool AH, bool BH, bool AREAL, int NI, int NJ>
+// WHOLE: kl is BK, without a test per 4 values; the body of nearly all
+// stages (chi = 512 ladder: 3.72 + 3.96 -> 3.66 + 3.87 ms per matvec stage,
+// chi = 96 sectors 0.717 + 0.778 -> 0.704 + 0.751 ms).
+template <class T, bool AH, bool BH, bool AREAL, int NI, int NJ, bool WHOLE = false>
 __device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, int j0, int kl) {
   const int lane = threadIdx.x & 31;
   const int gid = lane >> 2, tig = lane & 3;
@@ -199,7 +202,7 @@ __device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, 
   const int xk = (gid & 3) << 2, xt = tig << 2;  // the rows' XOR patterns
 #pragma unroll
   for (int kk = 0; kk < BK; kk += 4) {
-    if (kk >= kl) break;
+    if (!WHOLE && kk >= kl) break;
     double ar[NI], ai[NI], as[NI], br[NJ], bi[NJ];
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
@@ -302,11 +305,13 @@ zgemm_grouped_fp64(const GemmTile* __restrict__ tiles, const GemmTask* __restric
     // at most WI x WJ slices, one straight-line body each
     if (nj == 2) {
       if constexpr (T::WJ >= 2) {
-        if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 2>(c, sbuf, i0, j0, len0);
+        if (ni == 2 && len0 == BK) mma_stage<T, AH, BH, AREAL, 2, 2, true>(c, sbuf, i0, j0, len0);
+        else if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 2>(c, sbuf, i0, j0, len0);
         else mma_stage<T, AH, BH, AREAL, 1, 2>(c, sbuf, i0, j0, len0);
       }
     } else if (nj == 1) {
-      if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 1>(c, sbuf, i0, j0, len0);
+      if (ni == 2 && len0 == BK) mma_stage<T, AH, BH, AREAL, 2, 1, true>(c, sbuf, i0, j0, len0);
+      else if (ni == 2) mma_stage<T, AH, BH, AREAL, 2, 1>(c, sbuf, i0, j0, len0);
       else mma_stage<T, AH, BH, AREAL, 1, 1>(c, sbuf, i0, j0, len0);
     }
     since += len0;

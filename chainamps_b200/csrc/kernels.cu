@@ -327,8 +327,12 @@ k_maxpy_norm(const double* __restrict__ Vr, const double* __restrict__ Vi, int64
 // because a warp reduction per tile and vector took as long as the loads.
 // The partial sums are added by the last CTA to finish, in a fixed order.
 // Before (five passes, 8-byte loads): 3.0 to 4.2 TB/s of 16 (2 j + 13) n bytes,
-// 90 ms of a ladder step at chi = 512 and 121 ms of an Ising step at chi = 64;
-// now 4.7 to 5.1 TB/s of fewer bytes, 54 and 75 ms.
+// 90 ms of a ladder step at chi = 512 and 121 ms of an Ising step at chi = 64.
+// In three passes with the basis in ascending order: 54 and 75 ms.  U_j and
+// U_{j-1}, read for w', are first in the sums over the basis too, while the
+// CTA's tile of them is in L1 or L2, and `update` walks the tiles from the end,
+// where `mdot` stopped: 5.5 to 6 TB/s, mdot + update 47.7 -> 43.9 ms of the
+// ladder step and 0.588 -> 0.557 ms per step of the Ising one.
 template <bool V2>
 __device__ __forceinline__ double2 load2(const double* __restrict__ p, int64_t i, int64_t n) {
   if (V2) return i < n ? *reinterpret_cast<const double2*>(p + i) : double2{0.0, 0.0};
@@ -451,7 +455,7 @@ k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restri
       local_step(x[p].y, y[p].y, s, b, pr.y, pi.y, ar, ai, v[p].y, u[p].y);
     }
 #pragma unroll 2
-    for (int q = c0; q < c1; ++q) {
+    for (int q = c1 - 1; q >= c0; --q) {
       const double* vq = U + (int64_t)q * ldv;
       double2 t{0.0, 0.0};
 #pragma unroll
@@ -511,7 +515,8 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
   const double* up = j > 0 ? uj - ldv : uj;
   double nrm = 0.0;
   const int64_t tile = (int64_t)KR_THREADS * 2 * P;
-  for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
+  // from the end: what `mdot` read last may still be in L2
+  for (int64_t base = (n - 1) / tile * tile - (int64_t)blockIdx.x * tile; base >= 0; base -= (int64_t)gridDim.x * tile) {
     double2 x[P], y[P];
     const int64_t i0 = base + (int64_t)tid * 2;
 #pragma unroll
@@ -525,7 +530,7 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
       local_step(x[p].y, y[p].y, s, b, pr.y, pi.y, ar, ai, v.y, u.y);
     }
 #pragma unroll 2
-    for (int q = 0; q <= j; ++q) {
+    for (int q = j; q >= 0; --q) {
       const double* vq = U + (int64_t)q * ldv;
       const double2 h = hs[q];
       double2 v[P], u[P];

@@ -1239,6 +1239,10 @@ int Heff::add_projectors(const Planar& in, Planar& out, cudaStream_t st) {
 
 int Heff::apply_device(const double* din, double* dout, cudaStream_t st) {
   if (!whole()) return fail(CMPS_ERR_STATE, "matvec is sharded: use the theta-layout entry point");
+  if (is_split(precision) && split_reads_arpack(*this)) {
+    CMPS_TRY(apply_split_arpack(*this, din, y, st));
+    return unpack(y, dout, st);
+  }
   CMPS_TRY(pack(din, x, st));
   if (is_split(precision)) {
     CMPS_TRY(apply_split_stage(*this, 1, x, y, st));

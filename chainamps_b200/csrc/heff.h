@@ -280,6 +280,10 @@ int apply_split(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
 int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
 int split_reset_error(Heff& H, cudaStream_t st);
 int apply_split_stage(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
+// The folded tcgen05 form of a whole handle without projectors reads an
+// ARPACK-order vector itself; out in the theta layout.
+bool split_reads_arpack(const Heff& H);
+int apply_split_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st);
 int split_error(Heff& H);
 // The form of the handle's split operator (CMPS_FORM_*).
 int split_form(const Heff& H);

@@ -50,6 +50,10 @@ struct SplitState {
   void* d_theta_chunks = nullptr;
   void* d_theta_tiles = nullptr;
   int64_t n_theta_tiles = 0;
+  // ARPACK vector -> S1A: one allocation for the members, column starts, row map and tiles (whole handles)
+  void* d_arp = nullptr;
+  const void *d_arp_mems = nullptr, *d_arp_starts = nullptr, *d_arp_rows = nullptr, *d_arp_tiles = nullptr;
+  int64_t n_arp_tiles = 0;
   int* d_err = nullptr;
   int* h_err = nullptr;  // pinned
   tc::TcPlan p1, p2;
@@ -108,6 +112,62 @@ __global__ void __launch_bounds__(256) k_split_theta_t(const ThetaTile* __restri
       dst[o + plane] = v.y;
       dst[o + 2 * plane] = v.z;
       dst[o + 3 * plane] = v.w;
+    }
+  }
+}
+
+// ARPACK vector -> split S1A, without the planar theta in between.  An
+// ARPACK column holds the rows (sigma1, a0) of one middle charge, so neither
+// side needs a transpose: a warp takes one column and 64 values of a0, and
+// goes through the states of a class, whose entries stand side by side in the
+// column (the row map gives their places), so that the strided reads of one
+// state leave the next ones' in L1.
+// HBM bound: 16 bytes in and 8 (BF16) or 16 (TF32) out per entry.  Through the
+// planar theta it took two kernels and 56 or 64 bytes: chi = 512 ladder matvec in
+// BF16 1.65 -> 1.55 ms, chi = 201 in TF32 0.426 -> 0.413 ms.  The planar way stays
+// for vectors that are in the theta layout already (the eigensolver's) and for
+// projectors, which read the planar vector too.
+struct ArpMember {
+  int64_t dst, row;  // chunk (m, sigma1) of S1A; its first row in the row map
+};
+struct ArpTile {
+  int64_t col;                             // first column, into the column starts
+  int32_t mem, nmem, a0, rows, ld, first;  // first: the column's row of the S1A chunk
+  int32_t ncols, pad;
+};
+__device__ __forceinline__ void store_pair(uint16_t* p, uint16_t a, uint16_t b) {
+  *reinterpret_cast<uint32_t*>(p) = (uint32_t)a | (uint32_t)b << 16;
+}
+__device__ __forceinline__ void store_pair(float* p, float a, float b) {
+  *reinterpret_cast<float2*>(p) = make_float2(a, b);
+}
+template <class E>
+__global__ void __launch_bounds__(256) k_split_arpack(const ArpTile* __restrict__ tiles,
+                                                      const ArpMember* __restrict__ mems,
+                                                      const int64_t* __restrict__ starts,
+                                                      const int32_t* __restrict__ rows,
+                                                      const double2* __restrict__ arp, E* __restrict__ dst,
+                                                      int64_t plane) {
+  const ArpTile t = tiles[blockIdx.x];
+  const int j = threadIdx.x >> 5, a = t.a0 + 2 * (int)(threadIdx.x & 31);
+  grid_wait();  // up to here only the plan was read
+  if (j >= t.ncols || a >= t.rows) return;
+  const bool two = a + 1 < t.rows;
+  const double2* col = arp + starts[t.col + j];
+  E* out = dst + (int64_t)(t.first + j) * t.ld + a;
+#pragma unroll 4
+  for (int q = 0; q < t.nmem; ++q) {
+    const ArpMember m = mems[t.mem + q];
+    const int32_t* r = rows + m.row + a;
+    const double2 v = col[r[0]], w = two ? col[r[1]] : make_double2(0.0, 0.0);
+    E x[4], y[4];
+    split4(v.x, v.y, x, x + 1, x + 2, x + 3);
+    split4(w.x, w.y, y, y + 1, y + 2, y + 3);
+#pragma unroll
+    for (int p = 0; p < 4; ++p) {
+      E* o = out + m.dst + p * plane;
+      if (two) store_pair(o, x[p], y[p]);
+      else *o = x[p];
     }
   }
 }
@@ -309,6 +369,7 @@ void release_split(Heff* h) {
   if (s->buf) dfree(s->buf);
   if (s->d_theta_chunks) dfree(s->d_theta_chunks);
   if (s->d_theta_tiles) dfree(s->d_theta_tiles);
+  if (s->d_arp) dfree(s->d_arp);
   if (s->d_err) dfree(s->d_err);
   if (s->h_err) cudaFreeHost(s->h_err);
   delete s;
@@ -604,6 +665,63 @@ static int build_split(Heff& H, bool bf16) {
                          H.ctx->stream));
     }
   }
+  // ---- ARPACK vector -> S1A: the same images, read from the ARPACK columns ----
+  if (H.whole()) {
+    std::vector<ArpMember> mems;
+    std::vector<ArpTile> tiles;
+    std::vector<int64_t> starts, colbase(nm, 0);
+    std::vector<int32_t> rows(H.map_rowth.size());
+    for (int m = 0; m < nm; ++m) {
+      colbase[m] = (int64_t)starts.size();
+      starts.resize(starts.size() + th.ncols[m], -1);
+      const Heff::MapSec& sec = H.map_secs[m];
+      for (int64_t i = 0; i < sec.nrows; ++i) rows[sec.rowstart + H.map_rowth[sec.rowstart + i]] = (int32_t)i;
+    }
+    for (const Heff::MapCol& c : H.map_cols) {
+      if (c.start < 0 || c.start + H.map_secs[c.m].nrows > H.n_allowed)
+        return fail(CMPS_ERR_STATE, "wavefunction column outside the ARPACK vector");
+      starts[colbase[c.m] + c.colth] = c.start;
+    }
+    for (int m = 0; m < nm; ++m) {
+      if (!H.in_need[m]) continue;
+      for (const std::vector<int>& mem : H.cls_mem) {
+        if (th.rowoff[m][mem[0]] < 0) continue;
+        const int s = A0.find(r.sub(th.mq[m], H.sigq[mem[0]]));
+        const int32_t mem0 = (int32_t)mems.size(), dim = (int32_t)A0.sdim[s];
+        for (int s1 : mem) mems.push_back(ArpMember{s1a_chunk[{m, s1}], H.map_secs[m].rowstart + th.rowoff[m][s1]});
+        for (int s2 = 0; s2 < d; ++s2) {
+          if (th.coloff[m][s2] < 0) continue;
+          const int32_t cols = (int32_t)A2.sdim[A2.find(r.add(th.mq[m], H.sigq[s2]))];
+          for (int32_t c0 = 0; c0 < cols; c0 += 8) {
+            const int32_t nc = std::min(8, cols - c0);
+            const int64_t col = colbase[m] + th.coloff[m][s2] + c0;
+            for (int32_t j = 0; j < nc; ++j)
+              if (starts[col + j] < 0) return fail(CMPS_ERR_STATE, "wavefunction column without an ARPACK column");
+            for (int32_t a0 = 0; a0 < dim; a0 += 64)
+              tiles.push_back(ArpTile{col, mem0, (int32_t)mem.size(), a0, dim, (int32_t)S->ldS[s],
+                                      (int32_t)(S->coloff_pad[m][s2] + c0), nc, 0});
+          }
+        }
+      }
+    }
+    if (!tiles.empty() && tiles.size() <= 0x7fffffffull) {
+      auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+      const size_t b_mem = sizeof(ArpMember) * mems.size(), b_st = sizeof(int64_t) * starts.size(),
+                   b_row = sizeof(int32_t) * rows.size(), b_tile = sizeof(ArpTile) * tiles.size();
+      CMPS_CUDA(dmalloc(&S->d_arp, al(b_mem) + al(b_st) + al(b_row) + al(b_tile)));
+      char* p = (char*)S->d_arp;
+      auto put = [&](const void* src, size_t bytes, const void** dst) -> int {
+        *dst = p;
+        p += al(bytes);
+        return copy_wait((void*)*dst, src, bytes, cudaMemcpyHostToDevice, H.ctx->stream);
+      };
+      CMPS_TRY(put(mems.data(), b_mem, &S->d_arp_mems));
+      CMPS_TRY(put(starts.data(), b_st, &S->d_arp_starts));
+      CMPS_TRY(put(rows.data(), b_row, &S->d_arp_rows));
+      CMPS_TRY(put(tiles.data(), b_tile, &S->d_arp_tiles));
+      S->n_arp_tiles = (int64_t)tiles.size();
+    }
+  }
   // ---- stage 1 plan: C1[r_pad, a0'] = sum S1A[r_pad, a0] LPS[a0', a0] ----
   tc::TcPlan& p1 = S->p1;
   std::map<std::pair<int, int>, int32_t> amap1;
@@ -857,6 +975,26 @@ int apply_split_stage(Heff& H, int which, const Planar& in, Planar& out, cudaStr
     return launch_stage(*S, 1, out, st);
   }
   return launch_stage(*S, 2, out, st);
+}
+
+bool split_reads_arpack(const Heff& H) {
+  return H.split && !H.low_canonical && H.split->n_arp_tiles > 0 && H.proj_np == 0;
+}
+
+int apply_split_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st) {
+  const SplitState& S = *H.split;
+  CMPS_TRY(split_reset_error(H, st));
+  auto gather = [&](auto* dst) -> int {
+    using E = std::remove_pointer_t<decltype(dst)>;
+    CMPS_CUDA(launch_chained(k_split_arpack<E>, dim3((unsigned)S.n_arp_tiles), dim3(256), 0, st,
+                             (const ArpTile*)S.d_arp_tiles, (const ArpMember*)S.d_arp_mems,
+                             (const int64_t*)S.d_arp_starts, (const int32_t*)S.d_arp_rows, (const double2*)in, dst,
+                             S.s1a_len));
+    return CMPS_OK;
+  };
+  CMPS_TRY(S.bf16 ? gather((uint16_t*)S.at(S.s1a_off)) : gather(S.f32(S.s1a_off)));
+  CMPS_TRY(launch_stage(S, 1, out, st));
+  return launch_stage(S, 2, out, st);
 }
 
 int split_error(Heff& H) {

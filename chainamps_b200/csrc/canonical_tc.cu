@@ -122,6 +122,73 @@ __global__ void __launch_bounds__(256) k_gather_theta(const XinBlock* __restrict
   }
 }
 
+// ARPACK vector -> Theta_in, without the planar theta in between: the tiles of
+// Heff::pack (up to 32 columns of one (m, sigma2) x 64 rows of the ARPACK
+// columns), split on the way into shared memory and transposed there, since
+// Theta_in has a2 fastest.  A row's place comes from a table per (m, class of
+// sigma2).  HBM bound: 16 bytes in and 8 out per entry, 56 through the planar
+// theta, which stays for theta-layout vectors and for projectors.  chi = 128
+// Ising matvec 8.45 -> 8.29 ms.
+struct XinGroup {
+  int64_t row0;         // the row table of the group's (m, class of sigma2); below 0: no such block is read
+  int32_t col, pad;     // the group's first column in a row of Theta_in
+};
+constexpr int kArpLd = 65;
+__global__ void __launch_bounds__(256) k_gather_arpack(const Heff::PackTile* __restrict__ tiles,
+                                                       const Heff::PackGroup* __restrict__ groups,
+                                                       const int64_t* __restrict__ starts,
+                                                       const XinGroup* __restrict__ xin,
+                                                       const int64_t* __restrict__ rows,
+                                                       const double2* __restrict__ arp, uint16_t* __restrict__ dst,
+                                                       int64_t plane) {
+  __shared__ ushort4 t[32 * kArpLd];  // [column][row]
+  const Heff::PackTile tl = tiles[blockIdx.x];
+  const Heff::PackGroup g = groups[tl.group];
+  const XinGroup x = xin[tl.group];
+  const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;
+  const int nr = (int)min((int64_t)64, g.nrows - tl.r0), nc = (int)g.cnt;
+  grid_wait();  // up to here only the plan was read
+  if (x.row0 < 0) return;
+  double2 v[8];
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int j = ty + 8 * (k / 2), r = tx + 32 * (k % 2);
+    if (j < nc && r < nr) v[k] = arp[starts[g.off + j] + tl.r0 + r];
+  }
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int j = ty + 8 * (k / 2), r = tx + 32 * (k % 2);
+    if (j < nc && r < nr) {
+      ushort4 q;
+      split4(v[k].x, v[k].y, &q.x, &q.y, &q.z, &q.w);
+      t[j * kArpLd + r] = q;
+    }
+  }
+  __syncthreads();
+  const int c = 2 * (tx & 15);  // a pair of columns, two rows per warp
+#pragma unroll
+  for (int k = 0; k < 4; ++k) {
+    const int r = 2 * ty + (tx >> 4) + 16 * k;
+    if (r >= nr || c >= nc) continue;
+    const int64_t o = rows[x.row0 + tl.r0 + r];
+    if (o < 0) continue;
+    const ushort4 a = t[c * kArpLd + r];
+    uint16_t* p = dst + o + x.col + c;
+    if (c + 1 < nc) {
+      const ushort4 b = t[(c + 1) * kArpLd + r];
+      *reinterpret_cast<uint32_t*>(p) = (uint32_t)a.x | (uint32_t)b.x << 16;
+      *reinterpret_cast<uint32_t*>(p + plane) = (uint32_t)a.y | (uint32_t)b.y << 16;
+      *reinterpret_cast<uint32_t*>(p + 2 * plane) = (uint32_t)a.z | (uint32_t)b.z << 16;
+      *reinterpret_cast<uint32_t*>(p + 3 * plane) = (uint32_t)a.w | (uint32_t)b.w << 16;
+    } else {
+      p[0] = a.x;
+      p[plane] = a.y;
+      p[2 * plane] = a.z;
+      p[3 * plane] = a.w;
+    }
+  }
+}
+
 inline int64_t pad8(int64_t x) { return (x + 7) & ~int64_t(7); }
 inline int64_t align64(int64_t x) { return (x + 63) & ~int64_t(63); }
 
@@ -140,6 +207,8 @@ struct CanonTc {
   XinBlock* d_xin = nullptr;
   int n_xin = 0;
   int64_t max_runs = 0;
+  XinGroup* d_xgroups = nullptr;  // ARPACK vector -> Theta_in: one per group of Heff::pack, and the row tables
+  int64_t* d_xrows = nullptr;
   tc::TcPlan pR, pW2, pW1, pL;
   int* d_err = nullptr;
   int* h_err = nullptr;  // pinned
@@ -151,6 +220,8 @@ struct CanonTc {
     if (zv && own_zv) dfree(zv);
     if (y && own_y) dfree(y);
     if (d_xin) dfree(d_xin);
+    if (d_xgroups) dfree(d_xgroups);
+    if (d_xrows) dfree(d_xrows);
     if (d_err) dfree(d_err);
     if (h_err) cudaFreeHost(h_err);
   }
@@ -594,6 +665,48 @@ int build_canonical_tc(Heff& H) {
     CMPS_CUDA(dmalloc(&T->d_xin, sizeof(XinBlock) * xb.size()));
     CMPS_TRY(copy_wait(T->d_xin, xb.data(), sizeof(XinBlock) * xb.size(), cudaMemcpyHostToDevice, st));
   }
+  {
+    // the groups in the order of Heff::build_pack
+    std::vector<XinGroup> xg;
+    std::vector<int64_t> xr;
+    int64_t ntiles = 0;
+    for (int m = 0; m < nm; ++m) {
+      const Heff::MapSec& sec = H.map_secs[m];
+      std::vector<int64_t> row0(ncls, -1);
+      for (int c2 = 0; c2 < ncls; ++c2) {
+        if (ccoff[m][c2] < 0) continue;
+        std::vector<int64_t> at(sec.nrows, -1);  // by theta row
+        bool any = false;
+        for (int c1 = 0; c1 < ncls; ++c1) {
+          auto it = xoff.find({m, c1, c2});
+          if (it == xoff.end()) continue;
+          any = true;
+          const int64_t n1p = pad8(ncl(c1)), len = pad8(ncl(c2)) * pad8(ccdim[m][c2]);
+          for (int64_t i = 0; i < ncl(c1); ++i)
+            for (int64_t a0 = 0; a0 < rcdim[m][c1]; ++a0)
+              at[rcoff[m][c1] + i * rcdim[m][c1] + a0] = it->second + (a0 * n1p + i) * len;
+        }
+        if (!any) continue;
+        row0[c2] = (int64_t)xr.size();
+        for (int64_t i = 0; i < sec.nrows; ++i) xr.push_back(at[H.map_rowth[sec.rowstart + i]]);
+      }
+      for (int s2 = 0; s2 < H.d; ++s2) {
+        if (th.coloff[m][s2] < 0) continue;
+        const int c2 = H.cls_of[s2];
+        for (int64_t e0 = 0; e0 < ccdim[m][c2]; e0 += 32) {
+          xg.push_back(XinGroup{row0[c2], (int32_t)(H.cls_pos[s2] * pad8(ccdim[m][c2]) + e0), 0});
+          ntiles += (sec.nrows + 63) / 64;
+        }
+      }
+    }
+    if (ntiles != H.n_pack_tiles) return fail(CMPS_ERR_STATE, "canonical tcgen05 form: pack groups differ");
+    if (!xr.empty()) {
+      CMPS_CUDA(dmalloc(&T->d_xgroups, sizeof(XinGroup) * xg.size()));
+      CMPS_TRY(copy_wait(T->d_xgroups, xg.data(), sizeof(XinGroup) * xg.size(), cudaMemcpyHostToDevice, st));
+      CMPS_CUDA(dmalloc(&T->d_xrows, sizeof(int64_t) * xr.size()));
+      CMPS_TRY(copy_wait(T->d_xrows, xr.data(), sizeof(int64_t) * xr.size(), cudaMemcpyHostToDevice, st));
+    }
+  }
   CMPS_CUDA(dmalloc(&T->d_err, sizeof(int)));
   CMPS_CUDA(cudaMemsetAsync(T->d_err, 0, sizeof(int), st));
   CMPS_CUDA(cudaMallocHost(&T->h_err, sizeof(int)));
@@ -726,17 +839,8 @@ int build_canonical_tc(Heff& H) {
   return CMPS_OK;
 }
 
-// which: 1 = theta in, stages R and W2; 2 = stages W1 and L; 0 = all.
-int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st) {
-  CanonTc* T = H.ctc;
-  if (!T) return fail(CMPS_ERR_STATE, "canonical tcgen05 form not prepared");
+static int run_stages(CanonTc* T, int which, Planar& out, cudaStream_t st) {
   if (which != 2) {
-    if (T->n_xin > 0 && T->max_runs > 0) {
-      const int64_t gx = std::min<int64_t>((T->max_runs + 7) / 8, 2048);
-      k_gather_theta<<<dim3((unsigned)gx, (unsigned)T->n_xin), 256, 0, st>>>(T->d_xin, in.re(), in.im(), T->xin,
-                                                                             T->xin_len);
-      CMPS_CUDA(cudaGetLastError());
-    }
     CMPS_TRY(tc::launch(3, T->pR, (float*)T->zv, T->zv_len, nullptr, 0, nullptr, 0, T->d_err, st));
     CMPS_TRY(tc::launch(3, T->pW2, (float*)T->y, T->y_len, nullptr, 0, nullptr, 0, T->d_err, st));
   }
@@ -745,6 +849,29 @@ int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaSt
     CMPS_TRY(tc::launch(4, T->pL, nullptr, 0, out.re(), out.len, nullptr, 0, T->d_err, st));
   }
   return CMPS_OK;
+}
+
+// which: 1 = theta in, stages R and W2; 2 = stages W1 and L; 0 = all.
+int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st) {
+  CanonTc* T = H.ctc;
+  if (!T) return fail(CMPS_ERR_STATE, "canonical tcgen05 form not prepared");
+  if (which != 2 && T->n_xin > 0 && T->max_runs > 0) {
+    const int64_t gx = std::min<int64_t>((T->max_runs + 7) / 8, 2048);
+    k_gather_theta<<<dim3((unsigned)gx, (unsigned)T->n_xin), 256, 0, st>>>(T->d_xin, in.re(), in.im(), T->xin,
+                                                                           T->xin_len);
+    CMPS_CUDA(cudaGetLastError());
+  }
+  return run_stages(T, which, out, st);
+}
+
+bool canonical_tc_reads_arpack(const Heff& H) { return H.ctc && H.ctc->d_xrows; }
+
+int apply_canonical_tc_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st) {
+  CanonTc* T = H.ctc;
+  CMPS_CUDA(launch_chained(k_gather_arpack, dim3((unsigned)H.n_pack_tiles), dim3(256), 0, st, H.d_pack_tiles,
+                           H.d_pack_groups, H.d_pack_starts, T->d_xgroups, T->d_xrows, (const double2*)in, T->xin,
+                           T->xin_len));
+  return run_stages(T, 0, out, st);
 }
 
 double canonical_tc_flops(const Heff& H) { return H.ctc ? H.ctc->flops : 0.0; }

@@ -266,6 +266,8 @@ int build_canonical_tc(Heff& H);
 void release_canonical_tc(Heff* h);
 // which: 1 = theta in, stages R and W2; 2 = stages W1 and L; 0 = all four
 int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
+bool canonical_tc_reads_arpack(const Heff& H);
+int apply_canonical_tc_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st);
 void canonical_tc_error_words(const Heff& H, int** d_err, int** h_err);
 // executed complex flops of one matvec, padding included
 double canonical_tc_flops(const Heff& H);
@@ -280,8 +282,8 @@ int apply_split(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
 int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
 int split_reset_error(Heff& H, cudaStream_t st);
 int apply_split_stage(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
-// The folded tcgen05 form of a whole handle without projectors reads an
-// ARPACK-order vector itself; out in the theta layout.
+// The tcgen05 forms of a whole handle without projectors read an ARPACK-order
+// vector themselves; out in the theta layout.
 bool split_reads_arpack(const Heff& H);
 int apply_split_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st);
 int split_error(Heff& H);

@@ -978,12 +978,15 @@ int apply_split_stage(Heff& H, int which, const Planar& in, Planar& out, cudaStr
 }
 
 bool split_reads_arpack(const Heff& H) {
-  return H.split && !H.low_canonical && H.split->n_arp_tiles > 0 && H.proj_np == 0;
+  if (H.proj_np) return false;
+  if (H.low_canonical) return canonical_tc_reads_arpack(H);
+  return H.split && H.split->n_arp_tiles > 0;
 }
 
 int apply_split_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st) {
-  const SplitState& S = *H.split;
   CMPS_TRY(split_reset_error(H, st));
+  if (H.low_canonical) return apply_canonical_tc_arpack(H, in, out, st);
+  const SplitState& S = *H.split;
   auto gather = [&](auto* dst) -> int {
     using E = std::remove_pointer_t<decltype(dst)>;
     CMPS_CUDA(launch_chained(k_split_arpack<E>, dim3((unsigned)S.n_arp_tiles), dim3(256), 0, st,

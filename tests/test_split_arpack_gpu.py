@@ -1,7 +1,7 @@
-"""The folded tcgen05 matvec reads an ARPACK-order vector itself where no
-projector asks for the planar one.  Against the general way (a projector of
+"""The tcgen05 matvecs, folded and canonical, read an ARPACK-order vector
+themselves where no projector asks for the planar one.  Against the general way (a projector of
 weight 0 takes it): the same operands, so the same numbers, over sectors
-around the 64 rows and 8 columns of its tiles, odd sizes, classes of one and
+around the 64 rows and 8 or 32 columns of their tiles, odd sizes, classes of one and
 of several states and bonds whose sectors lie in any order."""
 import numpy as np
 import pytest
@@ -23,7 +23,7 @@ def _bond(rng, dims, shuffled):
 ])
 def test_reads_arpack_vector(left, right, charges, shuffled):
     from chainamps_b200 import (Context, TwoVertexComponents, models, CMPS_SPLIT_TF32, CMPS_SPLIT_BF16,
-                                CMPS_ORDER_FOLDED)
+                                CMPS_ORDER_FOLDED, CMPS_ORDER_CANONICAL, CMPS_FORM_CANONICAL_TC)
     rng = np.random.default_rng(len(left) + len(charges))
     d, D, rules = len(charges), 3, (0,)
     ch, bq = np.array(charges, np.int64).reshape(-1, 1), np.zeros((D, 1), np.int64)
@@ -34,10 +34,12 @@ def test_reads_arpack_vector(left, right, charges, shuffled):
     R = models.random_environment(rng, rules, br, bq, list(range(D)), right=True)
     ctx = Context(0)
     h = TwoVertexComponents(ctx, rules, L, models.mpo_tensor(ch, W, bq), R)
-    h.set_order(CMPS_ORDER_FOLDED)
     x = rng.standard_normal(h.n) + 1j * rng.standard_normal(h.n)
-    for precision in (CMPS_SPLIT_TF32, CMPS_SPLIT_BF16):
+    for order, precision in ((CMPS_ORDER_FOLDED, CMPS_SPLIT_TF32), (CMPS_ORDER_FOLDED, CMPS_SPLIT_BF16),
+                             (CMPS_ORDER_CANONICAL, CMPS_SPLIT_BF16)):
+        h.set_order(order)
         h.set_precision(precision)
+        assert (h.split_form() == CMPS_FORM_CANONICAL_TC) == (order == CMPS_ORDER_CANONICAL)
         got = h.multiply(x)
         h.set_projectors([x], [0.0])
         want = h.multiply(x)

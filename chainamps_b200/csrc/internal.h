@@ -216,7 +216,7 @@ struct GemmPlan {
 // Empirical tile-shape choice: `run` launches the plan once; every shape is
 // timed (one warm-up, three timed launches, CUDA events on st) and the
 // fastest kept.  Results are cached per process by plan signature (role,
-// task and term counts, flops, padded-work choice), so a plan of the same
+// task and term counts, flops, default choice), so a plan of the same
 // population is not timed again.
 struct TuneStats {
   int tuned = 0, cached = 0;

@@ -37,9 +37,13 @@
 //    filled by 8-byte cp.async (block offsets and leading dimensions have any
 //    parity) and one barrier per 16 values of K.
 // Before (64 x 64 tiles, four products, two CTAs per SM) and now, per matvec:
-// ladder at chi = 512 11.8 and 9.4 ms, Ising chains at chi = 64 10.8 and 5.7
-// ms, 40 uneven sectors 3.4 and 1.5 ms.  The DMMA pipe is 49 to 63% busy; the
-// rest goes to fragment and operand loads that the warps issue between DMMAs.
+// ladder at chi = 512 11.9 and 7.7 ms (the zero parts of T, which the plans now
+// leave out, are a fifth of that), Ising chains at chi = 64 10.9 and 6.0 ms, 40
+// uneven sectors 3.4 and 1.4 ms.  The DMMA pipe is 55 to 63% busy on ragged
+// blocks and 68 to 71% on blocks without remainders; a loop of this shape on
+// data in shared memory reaches 83%, 10% of it lost to the sums of P3, which
+// share the pipe.  The rest goes to operand loads and their addresses.
+// An infinite entry gives NaN where four products could give an infinity.
 //
 // An element's value does not depend on the tile shape or on how tasks are
 // cut: the order of its DMMAs and folds is fixed by its terms alone.

@@ -151,11 +151,11 @@ int cmps_heff_flops(const cmps_heff* h, double* canonical, double* executed);
 /* Measured tile shapes (no counterpart in the reference): every grouped GEMM
  * plan the handle's matvec runs (folded or canonical, FP64 or the FP32
  * canonical form; the tcgen05 split stages have fixed tiles) is launched
- * with each output tile shape -- 64x64, 32x128, 128x32 -- and keeps the
- * fastest.  Choices are cached per process by plan signature; `cached`
+ * with each output tile shape -- 32x32 and 32x16 in FP64, 64x64, 32x128 and
+ * 128x32 in FP32 -- and keeps the fastest.  Choices are cached per process by plan signature; `cached`
  * counts the plans that took a cached choice.  ms_heuristic / ms_best: the
- * summed per-launch times of the tuned plans with the padded-work choice and
- * with the measured one.  Outputs may be NULL. */
+ * summed per-launch times of the tuned plans with the default choice and with the
+ * measured one.  Outputs may be NULL. */
 int cmps_heff_autotune(cmps_heff* h, int* tuned, int* cached, double* ms_heuristic, double* ms_best);
 /* Chooses the contraction order of the FP64 matvec (CMPS_ORDER_*); no
  * counterpart in the reference, whose only order is the folded one. */
@@ -173,9 +173,10 @@ int cmps_heff_split_form(const cmps_heff* h, int* form);
  * would add an allocation and a device-wide synchronisation per iteration.
  * Same inputs and result as cmps_heff_apply_device (FP64 handles only), but
  * its scratch -- the gathered vector, the stage-1 intermediate and the
- * stage-2 output, 4 * n_allowed + 2 * |T| doubles -- lives in one static
- * device array of at most 32 MiB held by every GPU that loads the library;
- * larger problems are rejected with CMPS_ERR_ARG.  The first call on a device
+ * stage-2 output, 4 * n_allowed + 2 * |T| doubles, |T| counted with the rows
+ * and columns of T that are zero or unread -- lives in one static device array
+ * of at most 32 MiB held by every GPU that loads the library; larger problems
+ * are rejected with CMPS_ERR_ARG.  The first call on a device
  * looks up that array's device address (cudaGetSymbolAddress), so make the
  * first call before any stream capture.  All calls share the array: calls
  * that overlap on the GPU race.  Nothing in it needs to start at zero. */

@@ -5,6 +5,7 @@
 
 #include <map>
 #include <memory>
+#include <stdexcept>
 #include <vector>
 
 #include "internal.h"
@@ -35,6 +36,23 @@ struct ThetaSpace {
   int find(const QKey& q) const {
     auto it = mfind.find(q);
     return it == mfind.end() ? -1 : it->second;
+  }
+};
+
+// Offsets of blocks by key, in key order (they are added in it): a hundred
+// thousand of them on the Ising chains, where a tree's nodes took longer than
+// the blocks themselves.
+struct BlockOffsets : std::vector<std::pair<std::array<int, 4>, int64_t>> {
+  using Key = std::array<int, 4>;
+  const_iterator find(const Key& k) const {
+    auto it = std::lower_bound(begin(), end(), k, [](const value_type& a, const Key& b) { return a.first < b; });
+    return it != end() && it->first == k ? it : end();
+  }
+  size_t count(const Key& k) const { return find(k) != end(); }
+  int64_t at(const Key& k) const {
+    auto it = find(k);
+    if (it == end()) throw std::out_of_range("block offsets");
+    return it->second;
   }
 };
 
@@ -106,7 +124,7 @@ struct Heff {
   AxpyTerm* d_lp_terms = nullptr;
   AxpyBlock* d_rp_blocks = nullptr;
   AxpyTerm* d_rp_terms = nullptr;
-  std::map<std::array<int, 4>, int64_t> lp_off, rp_off;  // (b1, sigma', sigma, sector) -> offset
+  BlockOffsets lp_off, rp_off;  // (b1, sigma', sigma, sector) -> offset
   std::vector<int64_t> t_base;   // [b1 * nm + m] -> offset into T, -1 if no element is both produced and read
   std::vector<std::vector<uint8_t>> t_reads;  // [b1 * nm + m][sigma2]: stage 2 reads these columns of the block
   Planar T;                      // stage-1 intermediate, allocated on first use (ensure_T)

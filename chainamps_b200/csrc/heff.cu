@@ -819,7 +819,7 @@ int Heff::build_plans() {
   in_need.assign(nm, 0);
   // Dense (b, sigma', sigma, sector) -> block offset tables of lp_off /
   // rp_off for the plan loops below (several lookups per (b, m, sigma',
-  // sigma)), when they stay small; the maps otherwise.
+  // sigma)), when they stay small; searched otherwise.
   const int64_t nlp = (int64_t)D * d * d * A0.nsec(), nrp = (int64_t)D * d * d * A2.nsec();
   constexpr int64_t kDenseMax = int64_t(1) << 24;
   std::vector<int64_t> lp_tab, rp_tab;

@@ -1452,8 +1452,8 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     int k = 0;
     double beta0 = -1.0;
     bool split_used = false;
-    // Step j: y = H U_j, then the three passes of VecOps::lanczos.  The last
-    // step's vector is not part of the basis (x is free until the cycle ends).
+    // Step j: y = H U_j, then the three passes of VecOps::lanczos.  The vector
+    // after the last step's is not part of the basis and not stored.
     auto issue = [&](int j) -> int {
       cudaEvent_t* e = ev + 3 * (j & 1);
       Planar vj = view(j);
@@ -1465,8 +1465,8 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
         split_used = true;
       }
       CMPS_CUDA(cudaEventRecord(e[1], st));
-      double* out = j + 1 < kdim ? vre(j + 1) : x.re();
-      CMPS_TRY(ops.lanczos(kv.d, ldv, y.re(), y.im(), j, out, out + n, h_ab + 2 * (j & 1), st));
+      double* out = j + 1 < kdim ? vre(j + 1) : nullptr;
+      CMPS_TRY(ops.lanczos(kv.d, ldv, y.re(), y.im(), j, out, out ? out + n : nullptr, h_ab + 2 * (j & 1), st));
       CMPS_CUDA(cudaEventRecord(e[2], st));
       return CMPS_OK;
     };

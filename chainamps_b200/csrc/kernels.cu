@@ -493,9 +493,9 @@ k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restri
     for (int r = tid; r < 2 * (c1 - c0); r += KR_THREADS) c.h[2 * c0 + r] *= c.scale[c0 + r / 2];
 }
 
-// U_{j+1} = w' - sum_{i <= j} h_i s_i U_i into (or, oi); then the step's
-// coefficients, which the host reads from `host` (pinned) after the stream
-// has come this far.
+// U_{j+1} = w' - sum_{i <= j} h_i s_i U_i into (outr, outi), or nowhere if null
+// (a cycle's last step needs its norm only); then the step's coefficients,
+// which the host reads from `host` (pinned) after the stream has come this far.
 template <bool V2, int P>
 __global__ void __launch_bounds__(KR_THREADS, 2)
 k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __restrict__ yr,
@@ -551,8 +551,10 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
 #pragma unroll
     for (int p = 0; p < P; ++p) {
       const int64_t i = i0 + (int64_t)p * KR_THREADS * 2;
-      store2<V2>(outr, i, n, x[p]);
-      store2<V2>(outi, i, n, y[p]);
+      if (outr) {
+        store2<V2>(outr, i, n, x[p]);
+        store2<V2>(outi, i, n, y[p]);
+      }
       nrm += x[p].x * x[p].x + y[p].x * y[p].x + x[p].y * x[p].y + y[p].y * y[p].y;
     }
   }

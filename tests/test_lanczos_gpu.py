@@ -72,3 +72,27 @@ def test_lowest_eigenpair(left, right, krylov, mixed):
     assert (st["split_matvecs"] > 0) == mixed
     del h
     ctx.close()
+
+
+@pytest.mark.parametrize("mixed", [False, True])
+@pytest.mark.parametrize("left,right", [([1], [1]), ([1], [2]), ([1, 1], [1, 1])])
+def test_smallest_spaces(left, right, mixed):
+    """One and two entries: the Krylov space is the whole space, and with one
+    entry the first step is the last one too."""
+    from chainamps_b200 import Context, TwoVertexComponents, models, CMPS_FP64, CMPS_SPLIT_BF16
+    rng = np.random.default_rng(7 * sum(left) + sum(right))
+    A, B = [_hermitian(rng, n) for n in left], [_hermitian(rng, n) for n in right]
+    want = min(np.linalg.eigvalsh(a)[0] + np.linalg.eigvalsh(b)[0] for a, b in zip(A, B))
+    W = np.eye(2).reshape(1, 2, 1, 2).astype(np.complex128)
+    Wt = models.mpo_tensor(np.zeros((1, 1), np.int64), W, np.zeros((2, 1), np.int64))
+    ctx = Context(0)
+    h = TwoVertexComponents(ctx, (0,), _environment(A, left, 0, False), Wt, _environment(B, right, 1, True))
+    h.set_precision(CMPS_SPLIT_BF16 if mixed else CMPS_FP64)
+    e, v, _ = h.HED(tol=TOL, max_restarts=200)
+    scale = max(1.0, abs(want))
+    assert abs(e - want) <= 2 * TOL * scale
+    assert abs(np.linalg.norm(v) - 1.0) <= 1e-12
+    h.set_precision(CMPS_FP64)
+    assert np.linalg.norm(h.multiply(v) - e * v) <= 2 * TOL * scale
+    del h
+    ctx.close()

@@ -24,26 +24,26 @@
 //    and the slices of a tile are dealt out evenly over its four warps in
 //    the best of the arrangements 4 x 1, 2 x 2, 1 x 4 (GemmTile::cut).  The
 //    work then is 1.07 x, 1.13 x and 1.09 x the useful one.
-//  * Three multiplications per complex product.  With P1 = Ar Br, P2 = Ai Bi
-//    and P3 = (Ar + Ai)(Br + Bi), Re = P1 - P2 and Im = P3 - P1 - P2: 3 DMMAs
-//    per slice pair and k-step instead of 4 (the sums are one DADD per
-//    fragment).  P1, P2 and P3 are folded into the result every kFold values
-//    of K, so that rounding errors do not grow along all of K: against exact
-//    sums the error is 1.01 x that of the four-product chain at K = 128 and
-//    0.25 x at K = 2400; whole matvecs are 0.3 to 0.8 x as far off.
+//  * Four products per complex one, Re = Ar Br - Ai Bi and Im = Ar Bi + Ai Br,
+//    each component from its own terms alone.  Three multiplications (Im from
+//    (Ar + Ai)(Br + Bi) less the other two) would be a quarter fewer DMMAs, but
+//    leave the rounding error of the real products in an imaginary part that
+//    may be many orders smaller: with Im / Re = 1e-8 in both operands its
+//    relative error is 1e-7 instead of 1e-15, and eigenvectors whose phase is
+//    fixed are nearly real.  The sums are folded into the result every kFold
+//    values of K, so that rounding errors do not grow along all of K.
 //  * AREAL: a plan whose A operand has no imaginary part (the MPO blocks of
 //    real operators) needs two products, Ar Br and Ar Bi, and no folding.
 //  * Four CTAs of four warps per SM, each with a ring of three 16 KB stages
 //    filled by 8-byte cp.async (block offsets and leading dimensions have any
 //    parity) and one barrier per 16 values of K.
-// Before (64 x 64 tiles, four products, two CTAs per SM) and now, per matvec:
-// ladder at chi = 512 11.9 and 7.7 ms (the zero parts of T, which the plans now
-// leave out, are a fifth of that), Ising chains at chi = 64 10.9 and 6.0 ms, 40
-// uneven sectors 3.4 and 1.4 ms.  The DMMA pipe is 55 to 63% busy on ragged
-// blocks and 68 to 71% on blocks without remainders; a loop of this shape on
-// data in shared memory reaches 83%, 10% of it lost to the sums of P3, which
-// share the pipe.  The rest goes to operand loads and their addresses.
-// An infinite entry gives NaN where four products could give an infinity.
+// Against whole 64 x 64 tiles with two CTAs per SM, per matvec: ladder at chi =
+// 512 11.9 and 8.7 ms (the zero parts of T, which the plans leave out, are a
+// fifth of that), Ising chains at chi = 64 10.9 and 6.1 ms, 40 uneven sectors 3.4
+// and 1.56 ms.  The same kernel with three multiplications took 7.7, 5.8 and
+// 1.43 ms.  A loop of this shape on registers reaches 36.9 TFLOP/s, with
+// fragment reads from shared memory 36.1; the rest goes to operand loads,
+// their addresses and the slices that the busiest warp has more.
 //
 // An element's value does not depend on the tile shape or on how tasks are
 // cut: the order of its DMMAs and folds is fixed by its terms alone.
@@ -74,7 +74,7 @@ namespace {
 constexpr int BK = 16;
 constexpr int NTHREADS = 128;
 constexpr int STAGES = 3;
-constexpr int kFold = 128;  // values of K between two folds of the three products
+constexpr int kFold = 128;  // values of K between two folds of the products
 template <int BM_, int BN_, int WI_, int WJ_, int CTAS_>
 struct Tile {
   static constexpr int BM = BM_, BN = BN_, WI = WI_, WJ = WJ_, CTAS = CTAS_;
@@ -185,18 +185,18 @@ __host__ __device__ __forceinline__ void arrange(int sm, int sn, int& hm, int& h
   }
 }
 
-// A warp's accumulators: the result and, unless AREAL, the three products
-// since the last fold.
+// A warp's accumulators: the result and, unless AREAL, the sums since the last
+// fold, Ar Br, Ai Bi and Ar Bi + Ai Br.
 template <class T>
 struct Acc {
   double cr[T::WI][T::WJ][2], ci[T::WI][T::WJ][2];
-  double p1[T::WI][T::WJ][2], p2[T::WI][T::WJ][2], p3[T::WI][T::WJ][2];
+  double rr[T::WI][T::WJ][2], ii[T::WI][T::WJ][2], ri[T::WI][T::WJ][2];
 };
 
 // One stage of kl values of K for a warp's NI x NJ slices, straight-line.
 // WHOLE: kl is BK, without a test per 4 values; the body of nearly all
-// stages (chi = 512 ladder: 3.72 + 3.96 -> 3.66 + 3.87 ms per matvec stage,
-// chi = 96 sectors 0.717 + 0.778 -> 0.704 + 0.751 ms).
+// stages (chi = 512 ladder: 4.18 + 4.49 -> 4.13 + 4.45 ms per matvec stage,
+// chi = 96 sectors 0.804 + 0.772 -> 0.796 + 0.759 ms).
 template <class T, bool AH, bool BH, bool AREAL, int NI, int NJ, bool WHOLE = false>
 __device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, int j0, int kl) {
   const int lane = threadIdx.x & 31;
@@ -207,15 +207,12 @@ __device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, 
 #pragma unroll
   for (int kk = 0; kk < BK; kk += 4) {
     if (!WHOLE && kk >= kl) break;
-    double ar[NI], ai[NI], as[NI], br[NJ], bi[NJ];
+    double ar[NI], ai[NI], br[NJ], bi[NJ];
 #pragma unroll
     for (int i = 0; i < NI; ++i) {
       const int o = AH ? kk * T::BM + (((i0 + i) * 8 + gid) ^ xt) : 8 * i * BK + (kk ^ xk);
       ar[i] = sA[o];
-      if (!AREAL) {
-        ai[i] = AH ? -sA[o + T::PLANE_A] : sA[o + T::PLANE_A];
-        as[i] = ar[i] + ai[i];
-      }
+      if (!AREAL) ai[i] = AH ? -sA[o + T::PLANE_A] : sA[o + T::PLANE_A];
     }
 #pragma unroll
     for (int j = 0; j < NJ; ++j) {
@@ -223,19 +220,25 @@ __device__ __forceinline__ void mma_stage(Acc<T>& c, const double* buf, int i0, 
       br[j] = sB[o];
       bi[j] = BH ? -sB[o + T::PLANE_B] : sB[o + T::PLANE_B];
     }
+    // one product of all slice pairs after the other, the two that share an
+    // accumulator apart (pair by pair: chi = 512 ladder 8.78 ms instead of 8.69).
+    // One accumulator for Re (with -Ai) instead of two makes its chain twice as
+    // long: 40 sectors 1.65 ms instead of 1.56; four, one per product, spill.
+    auto products = [](double (&d)[T::WI][T::WJ][2], const double (&a)[NI], const double (&b)[NJ]) {
 #pragma unroll
-    for (int j = 0; j < NJ; ++j)
+      for (int j = 0; j < NJ; ++j)
 #pragma unroll
-      for (int i = 0; i < NI; ++i) {
-        if (AREAL) {
-          dmma(c.cr[i][j][0], c.cr[i][j][1], ar[i], br[j]);
-          dmma(c.ci[i][j][0], c.ci[i][j][1], ar[i], bi[j]);
-        } else {
-          dmma(c.p1[i][j][0], c.p1[i][j][1], ar[i], br[j]);
-          dmma(c.p2[i][j][0], c.p2[i][j][1], ai[i], bi[j]);
-          dmma(c.p3[i][j][0], c.p3[i][j][1], as[i], br[j] + bi[j]);
-        }
-      }
+        for (int i = 0; i < NI; ++i) dmma(d[i][j][0], d[i][j][1], a[i], b[j]);
+    };
+    if constexpr (AREAL) {
+      products(c.cr, ar, br);
+      products(c.ci, ar, bi);
+    } else {
+      products(c.rr, ar, br);
+      products(c.ri, ar, bi);
+      products(c.ii, ai, bi);
+      products(c.ri, ai, br);
+    }
   }
 }
 
@@ -276,7 +279,7 @@ zgemm_grouped_fp64(const GemmTile* __restrict__ tiles, const GemmTask* __restric
     for (int j = 0; j < T::WJ; ++j)
 #pragma unroll
       for (int e = 0; e < 2; ++e)
-        c.cr[i][j][e] = c.ci[i][j][e] = c.p1[i][j][e] = c.p2[i][j][e] = c.p3[i][j][e] = 0.0;
+        c.cr[i][j][e] = c.ci[i][j][e] = c.rr[i][j][e] = c.ii[i][j][e] = c.ri[i][j][e] = 0.0;
 
   // issue cursor over (term, k): fills stage buffer b and returns its values of K
   int it = task.t0, left = 0;
@@ -327,9 +330,9 @@ zgemm_grouped_fp64(const GemmTile* __restrict__ tiles, const GemmTask* __restric
         for (int j = 0; j < T::WJ; ++j)
 #pragma unroll
           for (int e = 0; e < 2; ++e) {
-            c.cr[i][j][e] += c.p1[i][j][e] - c.p2[i][j][e];
-            c.ci[i][j][e] += (c.p3[i][j][e] - c.p1[i][j][e]) - c.p2[i][j][e];
-            c.p1[i][j][e] = c.p2[i][j][e] = c.p3[i][j][e] = 0.0;
+            c.cr[i][j][e] += c.rr[i][j][e] - c.ii[i][j][e];
+            c.ci[i][j][e] += c.ri[i][j][e];
+            c.rr[i][j][e] = c.ii[i][j][e] = c.ri[i][j][e] = 0.0;
           }
     }
     len0 = len1;
@@ -405,13 +408,13 @@ int launch_zgemm_fp64(const GemmPlan& p, bool a_h, bool b_h, const Planar& A, co
 }
 
 // A tile's cost in SM cycles: its busiest warp's DMMAs (16 cycles each; two
-// or three per slice pair and 4 values of K) or the issue of its loads and
+// or four per slice pair and 4 values of K) or the issue of its loads and
 // fragment reads, whichever is more, plus what its epilogue takes.
 template <class T>
 static double tile_cost(int sm, int sn, double k4, double k16, bool a_real) {
   int hm, hn, wml;
   arrange<T>(sm, sn, hm, hn, wml);
-  return std::max(k4 * hm * hn * (a_real ? 32 : 48), 300.0 * k16) + 500.0;
+  return std::max(k4 * hm * hn * (a_real ? 32 : 64), 300.0 * k16) + 500.0;
 }
 
 template <class T>
@@ -433,12 +436,12 @@ static double task_cost(const GemmPlan& p, const GemmTask& t, int64_t* ntiles, d
 // Tile shape of a plan in FP64: 32 x 32, or 32 x 16 where the 32 x 32 tiles
 // are too few to fill the GPU evenly -- a launch takes the larger of the
 // tiles' summed cost over 148 SMs and the longest tile beside the others on
-// its SM.  32 x 16 reads each element of A more often, which costs it 8 to
-// 16% on plans of many tiles: ladder at chi = 512, 4.98 + 4.44 ms in 32 x 32
-// and 5.80 + 4.74 ms in 32 x 16; 40 uneven sectors, 0.72 + 0.77 and 0.79 +
-// 0.74 ms; XXZ chain at chi = 250, 24 + 52 and 20 + 34 us.  Larger tiles
-// (64 x 32, 32 x 64) leave room for two CTAs per SM only and lost to 32 x 32
-// on every plan measured, by 2 to 50%.
+// its SM.  32 x 16 reads each element of A more often, which costs it up to 23%
+// on plans of many tiles: both stages in 32 x 32 and in 32 x 16, ladder at chi =
+// 512 4.13 + 4.44 and 4.42 + 4.34 ms, 40 uneven sectors 0.79 + 0.91 and 0.82 +
+// 0.75 ms, XXZ chain at chi = 250 21 + 51 and 17 + 33 us.  Larger tiles (64 x 32,
+// 32 x 64) leave room for two CTAs per SM only and lost to 32 x 32 on nearly
+// every plan.
 template <class T>
 static double launch_cost(const GemmPlan& p) {
   double sum = 0.0, longest = 0.0;

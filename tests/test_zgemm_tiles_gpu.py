@@ -92,3 +92,64 @@ def test_folded_order_skips_zero_parts_of_t(seed):
         assert np.all(err <= (bound if prec == CMPS_FP64 else 2e-4 * np.max(np.abs(want)))), (prec, np.max(err))
         del h
     ctx.close()
+
+
+@pytest.mark.parametrize("turned", [False, True])
+@pytest.mark.parametrize("ratio", [1e-4, 1e-8, 1e-12])
+def test_small_component_keeps_its_accuracy(ratio, turned):
+    """Nearly real operands (imaginary parts `ratio` of the real ones), and a
+    vector turned by i: the small component of the result is as accurate as
+    the large one.  Re and Im of a product are bounded each by its own terms,
+    Re by |a||c| + |b||d| and Im by |a||d| + |b||c|, which is the product of
+    |a| + j|b| and |c| + j|d| with j^2 = 1; a matvec of such numbers is two
+    real ones, of the sums and of the differences of the two parts.  1500 u of
+    it as above."""
+    from chainamps_b200 import (Context, TwoVertexComponents, models, CMPS_ORDER_FOLDED, CMPS_ORDER_CANONICAL)
+    d, D, rules = 3, 3, (0,)
+    rng = np.random.default_rng(17)
+    dims = ([9, 33, 64, 130], [65, 8, 3, 97])
+    bl, br = _bond(dims[0]), _bond(dims[1])
+    ch, bq = np.zeros((d, 1), np.int64), np.zeros((D, 1), np.int64)
+    draw = lambda *s: rng.standard_normal(s) + 1j * ratio * rng.standard_normal(s)  # noqa: E731
+    W = draw(d, D, d, D)
+    L = models.random_environment(rng, rules, bl, bq, list(range(D)), right=False)
+    R = models.random_environment(rng, rules, br, bq, list(range(D)), right=True)
+    for t in (L, R):
+        t.values = draw(t.values.size)
+    lm, rm = _mats(L, bl.shape[0], D), _mats(R, br.shape[0], D)
+    ref = ob.BlockHeff(rules, ch, bl, br, bq, W, lm, rm)
+    x = draw(ref.n) * (1j if turned else 1.0)
+    want = ref.matvec(x)
+
+    def real_part(sign):
+        f = lambda a: (np.abs(a.real) + sign * np.abs(a.imag)).astype(np.complex128)  # noqa: E731
+        h = ob.BlockHeff(rules, ch, bl, br, bq, f(W), *[[None if m is None else f(m) for m in e] for e in (lm, rm)])
+        return h.matvec(f(x)).real
+    plus, minus = real_part(1.0), real_part(-1.0)
+    bound_re, bound_im = 750 * U * (plus + minus), 750 * U * (plus - minus)
+    ctx = Context(0)
+    h = TwoVertexComponents(ctx, rules, L, models.mpo_tensor(ch, W, bq), R)
+    for order in (CMPS_ORDER_FOLDED, CMPS_ORDER_CANONICAL):
+        h.set_order(order)
+        err = h.multiply(x) - want
+        assert np.all(np.abs(err.real) <= bound_re), (order, np.max(np.abs(err.real) / bound_re))
+        assert np.all(np.abs(err.imag) <= bound_im), (order, np.max(np.abs(err.imag) / bound_im))
+    del h
+    ctx.close()
+
+
+def test_infinite_component():
+    """One entry, x = inf + i, L = 2 + i, R = 1 - i: L x = inf + i inf and Re of
+    its product with R is inf + inf."""
+    from chainamps_b200 import Context, TwoVertexComponents, models
+    one, z = np.zeros((1, 1), np.int64), np.ones((1, 1, 1, 1), np.complex128)
+    rng, rules = np.random.default_rng(0), (0,)
+    L = models.random_environment(rng, rules, one, one, [0], right=False)
+    R = models.random_environment(rng, rules, one, one, [0], right=True)
+    L.values, R.values = np.array([2 + 1j]), np.array([1 - 1j])
+    ctx = Context(0)
+    h = TwoVertexComponents(ctx, rules, L, models.mpo_tensor(one, z, one), R)
+    got = h.multiply(np.array([complex(np.inf, 1.0)]))
+    assert got[0].real == np.inf
+    del h
+    ctx.close()

@@ -473,11 +473,11 @@ int build_canonical32(Heff& H) {
 
 // The low-precision canonical matvec: theta (FP64) -> FP32, the four stages
 // on FP32 planes with FP32 accumulation, the owned output sectors -> FP64.
-int apply_canonical32(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st) {
+int apply_canonical32(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st, const double* scale) {
   Canon* C = H.canon;
   if (!C || !C->have32) return fail(CMPS_ERR_STATE, "canonical-order FP32 operands not prepared");
   if (which != 2) {
-    CMPS_TRY(to_fp32(in.re(), in.im(), H.in_len, C->x32, st));
+    CMPS_TRY(to_fp32(in.re(), in.im(), H.in_len, C->x32, st, scale));
     CMPS_TRY(launch_cgemm_fp32(C->sL, C->L32, C->x32, C->xz32, st));
     CMPS_TRY(launch_cgemm_fp32(C->sW1, C->ops32, C->xz32, C->y32, st));
   }

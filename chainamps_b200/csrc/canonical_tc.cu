@@ -73,7 +73,8 @@ struct XinBlock {
 // even throughout; four such pairs in flight.
 template <bool V2>
 __device__ __forceinline__ void gather_row(const double* __restrict__ re, const double* __restrict__ im,
-                                           uint16_t* __restrict__ o, int64_t plane, int n, int d2, int d2p) {
+                                           double f, uint16_t* __restrict__ o, int64_t plane, int n, int d2,
+                                           int d2p) {
   const int lane = threadIdx.x & 31;
   constexpr int W = V2 ? 2 : 1;
   for (int e0 = lane * W; e0 < n; e0 += 4 * 32 * W) {
@@ -97,7 +98,7 @@ __device__ __forceinline__ void gather_row(const double* __restrict__ re, const 
       const int at = d2 == d2p ? e : e / d2 * d2p + e % d2;
       uint16_t p[4][W];
 #pragma unroll
-      for (int w = 0; w < W; ++w) split4(xr[q][w], xi[q][w], &p[0][w], &p[1][w], &p[2][w], &p[3][w]);
+      for (int w = 0; w < W; ++w) split4(f * xr[q][w], f * xi[q][w], &p[0][w], &p[1][w], &p[2][w], &p[3][w]);
 #pragma unroll
       for (int k = 0; k < 4; ++k) {
         if (V2) *reinterpret_cast<uint32_t*>(o + at + k * plane) = (uint32_t)p[k][0] | (uint32_t)p[k][W - 1] << 16;
@@ -109,16 +110,18 @@ __device__ __forceinline__ void gather_row(const double* __restrict__ re, const 
 
 __global__ void __launch_bounds__(256) k_gather_theta(const XinBlock* __restrict__ blocks,
                                                       const double* __restrict__ re, const double* __restrict__ im,
-                                                      uint16_t* __restrict__ dst, int64_t plane) {
+                                                      const double* __restrict__ scale, uint16_t* __restrict__ dst,
+                                                      int64_t plane) {
   const XinBlock b = blocks[blockIdx.y];
+  const double f = scale ? *scale : 1.0;
   const int rows = b.d0 * b.n1;
   const bool even = ((b.src | b.ncols | b.d2) & 1) == 0 && (((uintptr_t)re | (uintptr_t)im) & 15) == 0;
   for (int r = blockIdx.x * (blockDim.x >> 5) + (threadIdx.x >> 5); r < rows; r += gridDim.x * (blockDim.x >> 5)) {
     const int a0 = r / b.n1, i = r - a0 * b.n1;
     const int64_t s = b.src + ((int64_t)i * b.d0 + a0) * b.ncols;
     uint16_t* o = dst + b.dst + ((int64_t)a0 * b.n1p + i) * b.n2p * b.d2p;
-    if (even) gather_row<true>(re + s, im + s, o, plane, b.n2 * b.d2, b.d2, b.d2p);
-    else gather_row<false>(re + s, im + s, o, plane, b.n2 * b.d2, b.d2, b.d2p);
+    if (even) gather_row<true>(re + s, im + s, f, o, plane, b.n2 * b.d2, b.d2, b.d2p);
+    else gather_row<false>(re + s, im + s, f, o, plane, b.n2 * b.d2, b.d2, b.d2p);
   }
 }
 
@@ -852,12 +855,12 @@ static int run_stages(CanonTc* T, int which, Planar& out, cudaStream_t st) {
 }
 
 // which: 1 = theta in, stages R and W2; 2 = stages W1 and L; 0 = all.
-int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st) {
+int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st, const double* scale) {
   CanonTc* T = H.ctc;
   if (!T) return fail(CMPS_ERR_STATE, "canonical tcgen05 form not prepared");
   if (which != 2 && T->n_xin > 0 && T->max_runs > 0) {
     const int64_t gx = std::min<int64_t>((T->max_runs + 7) / 8, 2048);
-    k_gather_theta<<<dim3((unsigned)gx, (unsigned)T->n_xin), 256, 0, st>>>(T->d_xin, in.re(), in.im(), T->xin,
+    k_gather_theta<<<dim3((unsigned)gx, (unsigned)T->n_xin), 256, 0, st>>>(T->d_xin, in.re(), in.im(), scale, T->xin,
                                                                            T->xin_len);
     CMPS_CUDA(cudaGetLastError());
   }

@@ -205,10 +205,11 @@ int launch32_shape(const GemmPlan& p, const Planar32& A, const Planar32& B, Plan
 }
 
 __global__ void k_to_f32(const double* __restrict__ re, const double* __restrict__ im, int64_t n,
-                         float* __restrict__ ore, float* __restrict__ oim) {
+                         const double* __restrict__ scale, float* __restrict__ ore, float* __restrict__ oim) {
+  const double f = scale ? *scale : 1.0;
   for (int64_t e = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; e < n; e += (int64_t)gridDim.x * blockDim.x) {
-    ore[e] = (float)re[e];
-    oim[e] = (float)im[e];
+    ore[e] = (float)(f * re[e]);
+    oim[e] = (float)(f * im[e]);
   }
 }
 __global__ void k_to_f64(const float* __restrict__ re, const float* __restrict__ im, int64_t n,
@@ -251,10 +252,10 @@ int launch_cgemm_fp32(const GemmPlan& p, const Planar32& A, const Planar32& B, P
   }
 }
 
-int to_fp32(const double* re, const double* im, int64_t n, Planar32& out, cudaStream_t st) {
+int to_fp32(const double* re, const double* im, int64_t n, Planar32& out, cudaStream_t st, const double* scale) {
   if (n > out.len) return fail(CMPS_ERR_STATE, "FP32 conversion: destination too short");
   if (n == 0) return CMPS_OK;
-  k_to_f32<<<grid_for(n), 256, 0, st>>>(re, im, n, out.re(), out.im());
+  k_to_f32<<<grid_for(n), 256, 0, st>>>(re, im, n, scale, out.re(), out.im());
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }

@@ -1146,13 +1146,15 @@ int Heff::apply_theta_fp64(const Planar& in, Planar& out, cudaStream_t st) {
 }
 
 namespace {
-// h[2p], h[2p+1] = -w_p * c_p (c_p = <phi_p, x>), for the subtracting multi-axpy
+// h[2p], h[2p+1] = -w_p * c_p (c_p = <phi_p, x>, times *scale unless null), for
+// the subtracting multi-axpy
 __global__ void k_proj_coef(const double* __restrict__ c, const double* __restrict__ w, int np,
-                            double* __restrict__ h) {
+                            const double* __restrict__ scale, double* __restrict__ h) {
   const int p = threadIdx.x;
   if (p < np) {
-    h[2 * p] = -w[p] * c[2 * p];
-    h[2 * p + 1] = -w[p] * c[2 * p + 1];
+    const double f = scale ? -w[p] * *scale : -w[p];
+    h[2 * p] = f * c[2 * p];
+    h[2 * p + 1] = f * c[2 * p + 1];
   }
 }
 }  // namespace
@@ -1223,14 +1225,14 @@ int Heff::set_projectors_device(int np, const double* d_phi_arpack, const double
   return CMPS_OK;
 }
 
-int Heff::add_projectors(const Planar& in, Planar& out, cudaStream_t st) {
+int Heff::add_projectors(const Planar& in, Planar& out, cudaStream_t st, const double* scale) {
   if (!proj_np) return CMPS_OK;
   const int64_t n = th.total;
   // d_proj: weights [0, np), then c = <phi_p, x> (2 np) and |x|^2, then one
   // scratch norm; the coefficients are turned into -w_p c_p in place
   double* c = d_proj + proj_np;
   CMPS_TRY(ops.mdot_dev(proj.d, proj.d + n, 2 * n, proj_np, in.re(), in.im(), c, st));
-  k_proj_coef<<<1, 64, 0, st>>>(c, d_proj, proj_np, c);
+  k_proj_coef<<<1, 64, 0, st>>>(c, d_proj, proj_np, scale, c);
   CMPS_CUDA(cudaGetLastError());
   return ops.maxpy_norm_dev(proj.d, proj.d + n, 2 * n, proj_np, c, out.re(), out.im(), c + 2 * proj_np + 1, st);
 }
@@ -1452,21 +1454,24 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     int k = 0;
     double beta0 = -1.0;
     bool split_used = false;
-    // Step j: y = H U_j, then the three passes of VecOps::lanczos.  The vector
-    // after the last step's is not part of the basis and not stored.
+    // Step j: y = H U_j, or y = H V_j in split precision, whose operands have
+    // the range of 32 bits while U_j is of H's own size; then the three passes
+    // of VecOps::lanczos.  The vector after the last step's is not part of the
+    // basis and not stored.
     auto issue = [&](int j) -> int {
       cudaEvent_t* e = ev + 3 * (j & 1);
       Planar vj = view(j);
       CMPS_CUDA(cudaEventRecord(e[0], st));
-      if (all_fp64 || j == 0) {
-        CMPS_TRY(apply_theta_fp64(vj, y, st));
-      } else {
-        CMPS_TRY(apply_split_async(*this, vj, y, st));
+      const bool split = !all_fp64 && j > 0;
+      if (split) {
+        CMPS_TRY(apply_split_async(*this, vj, y, st, ops.lanczos_coef().scale + j));
         split_used = true;
+      } else {
+        CMPS_TRY(apply_theta_fp64(vj, y, st));
       }
       CMPS_CUDA(cudaEventRecord(e[1], st));
       double* out = j + 1 < kdim ? vre(j + 1) : nullptr;
-      CMPS_TRY(ops.lanczos(kv.d, ldv, y.re(), y.im(), j, out, out ? out + n : nullptr, h_ab + 2 * (j & 1), st));
+      CMPS_TRY(ops.lanczos(kv.d, ldv, y.re(), y.im(), split, j, out, out ? out + n : nullptr, h_ab + 2 * (j & 1), st));
       CMPS_CUDA(cudaEventRecord(e[2], st));
       return CMPS_OK;
     };

@@ -171,7 +171,8 @@ struct Heff {
   int set_projectors(int np, const double* host_arpack, const double* weights);
   // the same from device vectors phi_p = conj(P_p), ARPACK order, interleaved
   int set_projectors_device(int np, const double* d_phi_arpack, const double* weights);
-  int add_projectors(const Planar& in, Planar& out, cudaStream_t st);
+  // scale: a factor of `in` on the device, or null
+  int add_projectors(const Planar& in, Planar& out, cudaStream_t st, const double* scale = nullptr);
   double flops_canonical = 0.0, flops_executed = 0.0;
   // Contraction order of the FP64 matvec: folded (LeftPart / RightPart, the
   // two stages above) or canonical (L, W1, W2, R one index at a time,
@@ -276,14 +277,16 @@ void release_canonical(Heff* h);
 int apply_canonical(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
 // the same in FP32 (FP32 copies of the operands built by build_canonical32)
 int build_canonical32(Heff& H);
-int apply_canonical32(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
+int apply_canonical32(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st,
+                      const double* scale = nullptr);
 
 // The canonical order in split BF16 on tcgen05 (canonical_tc.cu): whole
 // vectors only (no windows, every sector owned).
 int build_canonical_tc(Heff& H);
 void release_canonical_tc(Heff* h);
 // which: 1 = theta in, stages R and W2; 2 = stages W1 and L; 0 = all four
-int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
+int apply_canonical_tc(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st,
+                       const double* scale = nullptr);
 bool canonical_tc_reads_arpack(const Heff& H);
 int apply_canonical_tc_arpack(Heff& H, const double* in, Planar& out, cudaStream_t st);
 void canonical_tc_error_words(const Heff& H, int** d_err, int** h_err);
@@ -297,7 +300,8 @@ int apply_split(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
 // The same matvec without a host synchronisation; a pipeline time-out is
 // recorded in the handle's error word, cleared by split_reset_error() and
 // read by split_error().
-int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st);
+// scale: a factor of `in` on the device, or null.
+int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st, const double* scale = nullptr);
 int split_reset_error(Heff& H, cudaStream_t st);
 int apply_split_stage(Heff& H, int which, const Planar& in, Planar& out, cudaStream_t st);
 // The tcgen05 forms of a whole handle without projectors read an ARPACK-order

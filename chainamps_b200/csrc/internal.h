@@ -241,7 +241,9 @@ int launch_zgemm_fp64(const GemmPlan& p, bool a_h, bool b_h, const Planar& A, co
 // FP32 grouped complex GEMM (cgemm_fp32.cu): the same plans as
 // launch_zgemm_fp64 without conjugated operands.
 int launch_cgemm_fp32(const GemmPlan& p, const Planar32& A, const Planar32& B, Planar32& C, cudaStream_t st);
-int to_fp32(const double* re, const double* im, int64_t n, Planar32& out, cudaStream_t st);
+// scale: a factor on the device, or null
+int to_fp32(const double* re, const double* im, int64_t n, Planar32& out, cudaStream_t st,
+            const double* scale = nullptr);
 int to_fp64(const Planar32& in, int64_t n, double* re, double* im, cudaStream_t st);
 int launch_block_axpy(const AxpyBlock* d_blocks, int nblocks, const AxpyTerm* d_terms,
                       const Planar& src, Planar& dst, cudaStream_t st, bool accumulate = false);

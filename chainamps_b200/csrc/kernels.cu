@@ -312,7 +312,7 @@ k_maxpy_norm(const double* __restrict__ Vr, const double* __restrict__ Vi, int64
 // ---- One Lanczos step in three passes ---------------------------------------
 // The basis is kept unnormalised: vector i is U_i = V_i / s_i with the scale
 // s_i = 1 / |U_i| on the device (LanczosCoef::scale), so that no pass only
-// rescales.  With y = H U_j and w = s_j y,
+// rescales.  With w = s_j y, y = H U_j, or w = y, y = H V_j (`unit`),
 //   dot     a = <V_j, w>
 //   mdot    w' = w - beta_{j-1} V_{j-1} - a V_j;  h_i = <V_i, w'>, i <= j
 //   update  U_{j+1} = w' - sum_i h_i V_i;  beta_j = |U_{j+1}|, alpha_j = a + h_j
@@ -379,14 +379,16 @@ __device__ __forceinline__ bool add_partials(const double* __restrict__ partial,
   return true;
 }
 
-// a = s_j^2 <U_j, y>
+// a = <s_j U_j, w>, scaled before the products: U_j and y have H's size, and
+// their squares are as large as a double needs to hold
 template <bool V2, int P>
 __global__ void __launch_bounds__(KR_THREADS, 2)
 k_lanczos_dot(const double* __restrict__ ur, const double* __restrict__ ui, const double* __restrict__ yr,
-              const double* __restrict__ yi, int64_t n, int j, LanczosCoef c, double* __restrict__ partial,
-              unsigned* __restrict__ count) {
+              const double* __restrict__ yi, int64_t n, bool unit, int j, LanczosCoef c,
+              double* __restrict__ partial, unsigned* __restrict__ count) {
   __shared__ double red[2][KR_THREADS / 32];
   grid_wait();
+  const double su = c.scale[j], sy = unit ? 1.0 : su;
   double sr = 0.0, si = 0.0;
   const int64_t tile = (int64_t)KR_THREADS * 2 * P;
   for (int64_t base = (int64_t)blockIdx.x * tile; base < n; base += (int64_t)gridDim.x * tile) {
@@ -401,6 +403,8 @@ k_lanczos_dot(const double* __restrict__ ur, const double* __restrict__ ui, cons
     }
 #pragma unroll
     for (int p = 0; p < P; ++p) {
+      a[p].x *= su, a[p].y *= su, b[p].x *= su, b[p].y *= su;
+      x[p].x *= sy, x[p].y *= sy, y[p].x *= sy, y[p].y *= sy;
       sr += a[p].x * x[p].x + b[p].x * y[p].x + a[p].y * x[p].y + b[p].y * y[p].y;
       si += a[p].x * y[p].x - b[p].x * x[p].x + a[p].y * y[p].y - b[p].y * x[p].y;
     }
@@ -417,21 +421,21 @@ k_lanczos_dot(const double* __restrict__ ur, const double* __restrict__ ui, cons
     for (int w = 0; w < KR_THREADS / 32; ++w) t += red[threadIdx.x][w];
     partial[(int64_t)threadIdx.x * gridDim.x + blockIdx.x] = t;
   }
-  if (add_partials(partial, 2, c.a, count) && threadIdx.x < 2) c.a[threadIdx.x] *= c.scale[j] * c.scale[j];
+  add_partials(partial, 2, c.a, count);
 }
 
 // h_i = s_i <U_i, w'> for c0 <= i < c1; U_i at U + i ldv (re; im n further)
 template <bool V2, int P>
 __global__ void __launch_bounds__(KR_THREADS, 2)
 k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restrict__ yr,
-               const double* __restrict__ yi, int64_t n, int j, int c0, int c1, LanczosCoef c,
+               const double* __restrict__ yi, int64_t n, bool unit, int j, int c0, int c1, LanczosCoef c,
                double* __restrict__ partial, unsigned* __restrict__ count) {
   extern __shared__ double2 dots[];  // [c1 - c0][KR_THREADS]
   const int tid = threadIdx.x;
   grid_wait();
   for (int i = 0; i < c1 - c0; ++i) dots[i * KR_THREADS + tid] = double2{0.0, 0.0};
-  const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
-  const double ar = c.a[0] * s, ai = c.a[1] * s;
+  const double s = unit ? 1.0 : c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
+  const double ar = c.a[0] * c.scale[j], ai = c.a[1] * c.scale[j];
   const double* uj = U + (int64_t)j * ldv;
   const double* up = j > 0 ? uj - ldv : uj;
   const int64_t tile = (int64_t)KR_THREADS * 2 * P;
@@ -499,7 +503,7 @@ k_lanczos_mdot(const double* __restrict__ U, int64_t ldv, const double* __restri
 template <bool V2, int P>
 __global__ void __launch_bounds__(KR_THREADS, 2)
 k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __restrict__ yr,
-                 const double* __restrict__ yi, int64_t n, int j, double* __restrict__ outr,
+                 const double* __restrict__ yi, int64_t n, bool unit, int j, double* __restrict__ outr,
                  double* __restrict__ outi, LanczosCoef c, double* __restrict__ partial,
                  unsigned* __restrict__ count, double* __restrict__ host) {
   __shared__ double2 hs[128];
@@ -508,8 +512,8 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
   grid_wait();
   for (int i = tid; i <= j; i += KR_THREADS)
     hs[i] = double2{c.h[2 * i] * c.scale[i], c.h[2 * i + 1] * c.scale[i]};
-  const double s = c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
-  const double ar = c.a[0] * s, ai = c.a[1] * s;
+  const double s = unit ? 1.0 : c.scale[j], b = j > 0 ? c.beta[j - 1] * c.scale[j - 1] : 0.0;
+  const double ar = c.a[0] * c.scale[j], ai = c.a[1] * c.scale[j];
   __syncthreads();
   const double* uj = U + (int64_t)j * ldv;
   const double* up = j > 0 ? uj - ldv : uj;
@@ -735,37 +739,37 @@ LanczosCoef VecOps::lanczos_coef() const {
 // Tiles of 512 or 2048 elements: the small ones spread a short vector (the
 // XXZ chain's few thousand entries) over more CTAs; two CTAs per SM at most.
 template <bool V2, int P>
-static int lanczos_step(const VecOps& o, const double* U, int64_t ldv, const double* yr, const double* yi, int j,
-                        double* outr, double* outi, double* host, cudaStream_t st) {
+static int lanczos_step(const VecOps& o, const double* U, int64_t ldv, const double* yr, const double* yi, bool unit,
+                        int j, double* outr, double* outi, double* host, cudaStream_t st) {
   const LanczosCoef c = o.lanczos_coef();
   const int64_t tiles = (o.n + (int64_t)KR_THREADS * 2 * P - 1) / ((int64_t)KR_THREADS * 2 * P);
   const int g = (int)std::max<int64_t>(1, std::min<int64_t>(std::min(o.nb, 296), tiles));
   const double* uj = U + (int64_t)j * ldv;
-  CMPS_CUDA(launch_chained(k_lanczos_dot<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, uj, uj + o.n, yr, yi, o.n, j, c,
+  CMPS_CUDA(launch_chained(k_lanczos_dot<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, uj, uj + o.n, yr, yi, o.n, unit, j, c,
                            o.d_partial, o.d_count));
   constexpr int kChunk = 24;  // vectors per launch of the products: 96 KB of partial sums
   CMPS_TRY(ensure_smem_optin((const void*)k_lanczos_mdot<V2, P>, kChunk * KR_THREADS * (int)sizeof(double2)));
   for (int c0 = 0; c0 <= j; c0 += kChunk) {
     const int c1 = std::min(j + 1, c0 + kChunk);
     CMPS_CUDA(launch_chained(k_lanczos_mdot<V2, P>, dim3(g), dim3(KR_THREADS),
-                             (size_t)(c1 - c0) * KR_THREADS * sizeof(double2), st, U, ldv, yr, yi, o.n, j, c0, c1, c,
+                             (size_t)(c1 - c0) * KR_THREADS * sizeof(double2), st, U, ldv, yr, yi, o.n, unit, j, c0, c1, c,
                              o.d_partial, o.d_count));
   }
-  CMPS_CUDA(launch_chained(k_lanczos_update<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, U, ldv, yr, yi, o.n, j, outr,
+  CMPS_CUDA(launch_chained(k_lanczos_update<V2, P>, dim3(g), dim3(KR_THREADS), 0, st, U, ldv, yr, yi, o.n, unit, j, outr,
                            outi, c, o.d_partial, o.d_count, host));
   return CMPS_OK;
 }
 
-int VecOps::lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, int j, double* outr,
+int VecOps::lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, bool unit, int j, double* outr,
                     double* outi, double* host, cudaStream_t st) {
   if (j < 0 || j > 126) return fail(CMPS_ERR_ARG, "krylov dimension above 127");
   const bool even = n % 2 == 0 && ldv % 2 == 0 &&
                     (((uintptr_t)U | (uintptr_t)yr | (uintptr_t)yi | (uintptr_t)outr | (uintptr_t)outi) & 15) == 0;
   const bool wide = n >= (int64_t)148 * 2 * 2048;
-  if (even && wide) return lanczos_step<true, 4>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
-  if (even) return lanczos_step<true, 1>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
-  if (wide) return lanczos_step<false, 4>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
-  return lanczos_step<false, 1>(*this, U, ldv, yr, yi, j, outr, outi, host, st);
+  if (even && wide) return lanczos_step<true, 4>(*this, U, ldv, yr, yi, unit, j, outr, outi, host, st);
+  if (even) return lanczos_step<true, 1>(*this, U, ldv, yr, yi, unit, j, outr, outi, host, st);
+  if (wide) return lanczos_step<false, 4>(*this, U, ldv, yr, yi, unit, j, outr, outi, host, st);
+  return lanczos_step<false, 1>(*this, U, ldv, yr, yi, unit, j, outr, outi, host, st);
 }
 
 int VecOps::scale_dev(const double* xr, const double* xi, const double* d_s, bool inv_sqrt, double* yr, double* yi,

@@ -49,11 +49,11 @@ struct VecOps {
                      double* wi, double* d_nrm2, cudaStream_t st);
   // Step j of a Lanczos cycle with full re-orthogonalisation (kernels.cu):
   // basis vectors U_0 .. U_j at U + i ldv (real plane, imaginary plane n
-  // further), y = H U_j; the next vector into (outr, outi) unless they are null,
+  // further), y = H U_j, or H V_j where `unit` is set; the next vector into (outr, outi) unless they are null,
   // alpha_j and beta_j into host[0..1] (pinned memory) once the stream has come
   // this far.  The cycle's first scale, lanczos_coef().scale[0], is the caller's.
-  int lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, int j, double* outr, double* outi,
-              double* host, cudaStream_t st);
+  int lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, bool unit, int j, double* outr,
+              double* outi, double* host, cudaStream_t st);
   LanczosCoef lanczos_coef() const;
   unsigned* d_count = nullptr;  // CTAs of the current launch that have finished
   // y = s x with s = *d_s, or s = 1 / sqrt(*d_s) when inv_sqrt.

@@ -86,8 +86,10 @@ template <class E>
 __global__ void __launch_bounds__(256) k_split_theta_t(const ThetaTile* __restrict__ tiles,
                                                        const ThetaChunk* __restrict__ chunks,
                                                        const double* __restrict__ re, const double* __restrict__ im,
-                                                       E* __restrict__ dst, int64_t plane) {
+                                                       const double* __restrict__ scale, E* __restrict__ dst,
+                                                       int64_t plane) {
   __shared__ Quad<E> t[32][33];
+  const double f = scale ? *scale : 1.0;
   const ThetaTile tl = tiles[blockIdx.x];
   const ThetaChunk c = chunks[tl.chunk];
   const int tx = threadIdx.x & 31, ty = threadIdx.x >> 5;  // 32 x 8
@@ -97,7 +99,7 @@ __global__ void __launch_bounds__(256) k_split_theta_t(const ThetaTile* __restri
     if (r < c.rows && col < c.cols) {
       const int64_t o = c.src_off + (int64_t)r * c.src_ld + col;
       Quad<E> v;
-      split4(re[o], im[o], &v.x, &v.y, &v.z, &v.w);
+      split4(f * re[o], f * im[o], &v.x, &v.y, &v.z, &v.w);
       t[ty + 8 * k][tx] = v;
     }
   }
@@ -899,15 +901,15 @@ static int launch_stage(const SplitState& S, int which, Planar& out, cudaStream_
   return tc::launch(2, S.p2, nullptr, 0, out.re(), out.len, S.f32(S.ts_off), S.ts_len, S.d_err, st);
 }
 
-static int split_theta(const SplitState& S, const Planar& in, cudaStream_t st) {
+static int split_theta(const SplitState& S, const Planar& in, cudaStream_t st, const double* scale = nullptr) {
   if (S.n_theta_tiles == 0) return CMPS_OK;
   if (S.bf16)
     k_split_theta_t<uint16_t><<<(unsigned)S.n_theta_tiles, 256, 0, st>>>(
-        (const ThetaTile*)S.d_theta_tiles, (const ThetaChunk*)S.d_theta_chunks, in.re(), in.im(),
+        (const ThetaTile*)S.d_theta_tiles, (const ThetaChunk*)S.d_theta_chunks, in.re(), in.im(), scale,
         (uint16_t*)S.at(S.s1a_off), S.s1a_len);
   else
     k_split_theta_t<float><<<(unsigned)S.n_theta_tiles, 256, 0, st>>>(
-        (const ThetaTile*)S.d_theta_tiles, (const ThetaChunk*)S.d_theta_chunks, in.re(), in.im(),
+        (const ThetaTile*)S.d_theta_tiles, (const ThetaChunk*)S.d_theta_chunks, in.re(), in.im(), scale,
         S.f32(S.s1a_off), S.s1a_len);
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
@@ -936,20 +938,20 @@ int split_reset_error(Heff& H, cudaStream_t st) {
   return CMPS_OK;
 }
 
-int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st) {
+int apply_split_async(Heff& H, const Planar& in, Planar& out, cudaStream_t st, const double* scale) {
   if (H.low_canonical) {
     if (H.ctc)
-      CMPS_TRY(apply_canonical_tc(H, 0, in, out, st));
+      CMPS_TRY(apply_canonical_tc(H, 0, in, out, st, scale));
     else
-      CMPS_TRY(apply_canonical32(H, 0, in, out, st));
-    return H.add_projectors(in, out, st);
+      CMPS_TRY(apply_canonical32(H, 0, in, out, st, scale));
+    return H.add_projectors(in, out, st, scale);
   }
   SplitState* S = H.split;
   if (!S) return fail(CMPS_ERR_STATE, "split-precision operands not prepared");
-  CMPS_TRY(split_theta(*S, in, st));
+  CMPS_TRY(split_theta(*S, in, st, scale));
   CMPS_TRY(launch_stage(*S, 1, out, st));
   CMPS_TRY(launch_stage(*S, 2, out, st));
-  return H.add_projectors(in, out, st);
+  return H.add_projectors(in, out, st, scale);
 }
 
 // theta-space matvec in split precision: FP64 planar in -> FP64 planar out.

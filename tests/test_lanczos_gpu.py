@@ -96,3 +96,38 @@ def test_smallest_spaces(left, right, mixed):
     assert np.linalg.norm(h.multiply(v) - e * v) <= 2 * TOL * scale
     del h
     ctx.close()
+
+
+@pytest.mark.parametrize("size,precision,canonical", [
+    (1e120, "CMPS_FP64", False), (1e25, "CMPS_SPLIT_BF16", False), (1e25, "CMPS_SPLIT_TF32", False),
+    (1e25, "CMPS_SPLIT_BF16", True), (1e25, "CMPS_SPLIT_TF32", True)])
+@pytest.mark.parametrize("projected", [False, True])
+def test_large_operators(size, precision, canonical, projected):
+    """H of a size whose square still fits its format (64 bits, or the 32 of the
+    split forms' operands), with and without a projector that lifts the
+    ground state above the first excited one; tolerances as above."""
+    import chainamps_b200 as ca
+    from chainamps_b200 import models
+    rng = np.random.default_rng(5)
+    left, right = [13, 9], [11, 6]
+    A, B = [[size * _hermitian(rng, n) for n in dims] for dims in (left, right)]
+    levels = np.sort(np.concatenate([np.add.outer(np.linalg.eigvalsh(a), np.linalg.eigvalsh(b)).ravel()
+                                     for a, b in zip(A, B)]))
+    W = np.eye(2).reshape(1, 2, 1, 2).astype(np.complex128)
+    Wt = models.mpo_tensor(np.zeros((1, 1), np.int64), W, np.zeros((2, 1), np.int64))
+    ctx = ca.Context(0)
+    h = ca.TwoVertexComponents(ctx, (0,), _environment(A, left, 0, False), Wt, _environment(B, right, 1, True))
+    if canonical:
+        h.set_order(ca.CMPS_ORDER_CANONICAL)
+    if projected:
+        _, ground, _ = h.HED(tol=TOL, max_restarts=200)
+        h.set_projectors([ground.conj()], [2.0 * (levels[1] - levels[0])])
+    want = levels[1 if projected else 0]
+    h.set_precision(getattr(ca, precision))
+    e, v, _ = h.HED(tol=TOL, max_restarts=200, krylov_dim=40)
+    assert abs(e - want) <= 4 * TOL * abs(want)
+    assert abs(np.linalg.norm(v) - 1.0) <= 1e-12
+    h.set_precision(ca.CMPS_FP64)
+    assert np.linalg.norm(h.multiply(v) - e * v) <= 2 * TOL * abs(want)
+    del h
+    ctx.close()

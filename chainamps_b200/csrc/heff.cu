@@ -1475,9 +1475,17 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
       CMPS_CUDA(cudaEventRecord(e[2], st));
       return CMPS_OK;
     };
+    // the matvec of step j, which has run
+    auto count_matvec = [&](int j) -> int {
+      float ms = 0.f;
+      CMPS_CUDA(cudaEventElapsedTime(&ms, ev[3 * (j & 1)], ev[3 * (j & 1) + 1]));
+      const bool fp64 = all_fp64 || j == 0;
+      ++(fp64 ? eig_stats.mv_fp64 : eig_stats.mv_split);
+      (fp64 ? eig_stats.ms_fp64 : eig_stats.ms_split) += ms;
+      return CMPS_OK;
+    };
     int issued = 0;
     for (int j = 0; j < kdim; ++j) {
-      const bool fp64 = all_fp64 || j == 0;
       // Short vectors: the next step is issued before this one's coefficients
       // are read (it needs them on the device only), so that the GPU does not
       // wait for the host's turn, 40 us or so.  A cycle that ends at this step
@@ -1487,15 +1495,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
       cudaEvent_t* e = ev + 3 * (j & 1);
       CMPS_CUDA(cudaEventSynchronize(e[2]));
       ++nmv;
-      float mv_ms = 0.f;
-      CMPS_CUDA(cudaEventElapsedTime(&mv_ms, e[0], e[1]));
-      if (fp64) {
-        ++eig_stats.mv_fp64;
-        eig_stats.ms_fp64 += mv_ms;
-      } else {
-        ++eig_stats.mv_split;
-        eig_stats.ms_split += mv_ms;
-      }
+      CMPS_TRY(count_matvec(j));
       const double a = h_ab[2 * (j & 1)], b = h_ab[2 * (j & 1) + 1];
       al.push_back(a);
       be.push_back(b);
@@ -1541,6 +1541,10 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     CMPS_TRY(ops.combine(kv.d, kv.d + n, ldv, k, ycoef.data(), x.re(), x.im(), st));
     CMPS_TRY(ops.mdot_dev(nullptr, nullptr, 0, 0, x.re(), x.im(), nrm, st));
     CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, true, x.re(), x.im(), st));
+    if (issued > k) {  // a step issued ahead and dropped: its matvec has run all the same
+      CMPS_CUDA(cudaEventSynchronize(ev[3 * (k & 1) + 1]));
+      CMPS_TRY(count_matvec(k));
+    }
   }
   CMPS_CUDA(cudaEventRecord(ev[7], st));
   // HED post-processing (DMRG_routines.cpp:870-889)

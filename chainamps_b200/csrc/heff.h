@@ -202,7 +202,8 @@ struct Heff {
   int kv_dim = 0;
   VecOps ops;
   double* h_ab = nullptr;        // pinned: alpha_j, beta_j of the current Lanczos step
-  // Work of the last eigs() call.
+  // Work of the last eigs() call: every matvec that ran, also those of steps
+  // that were issued ahead and then dropped.
   struct EigStats {
     int mv_split = 0, mv_fp64 = 0, cycles = 0;
     double ms_split = 0.0, ms_fp64 = 0.0, ms_total = 0.0;

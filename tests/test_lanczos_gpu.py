@@ -131,3 +131,23 @@ def test_large_operators(size, precision, canonical, projected):
     assert np.linalg.norm(h.multiply(v) - e * v) <= 2 * TOL * abs(want)
     del h
     ctx.close()
+
+
+def test_stats_count_dropped_steps():
+    """A short vector's cycle that ends before its last step has issued one step
+    more, whose matvec is part of the solve's time and of its counts."""
+    from chainamps_b200 import Context, TwoVertexComponents, models
+    rng = np.random.default_rng(3)
+    left, right, krylov = [13, 9], [11, 6], 60
+    A, B = [_hermitian(rng, n) for n in left], [_hermitian(rng, n) for n in right]
+    W = np.eye(2).reshape(1, 2, 1, 2).astype(np.complex128)
+    Wt = models.mpo_tensor(np.zeros((1, 1), np.int64), W, np.zeros((2, 1), np.int64))
+    ctx = Context(0)
+    h = TwoVertexComponents(ctx, (0,), _environment(A, left, 0, False), Wt, _environment(B, right, 1, True))
+    _, _, applications = h.HED(tol=TOL, max_restarts=200, krylov_dim=krylov)
+    st = h.eigs_stats()
+    assert st["cycles"] == 1 and applications < krylov
+    assert st["fp64_matvecs"] == applications + 1
+    assert st["ms_fp64"] <= st["ms_total"]
+    del h
+    ctx.close()

@@ -1439,7 +1439,9 @@ int sweep_fidelity(Heff& H, const SvdResult& s, const std::vector<double>& lam, 
         }
       }
   }
-  *out = 1.0 - std::hypot(total_re, total_im);
+  // two unit vectors: an overlap above 1 is rounding, and the fidelity then 0
+  const double f = 1.0 - std::hypot(total_re, total_im);
+  *out = f < 0.0 ? 0.0 : f;
   return CMPS_OK;
 }
 

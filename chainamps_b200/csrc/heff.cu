@@ -977,6 +977,23 @@ int Heff::build_plans() {
       if (m >= 0 && t_base[(size_t)b1 * nm + m] >= 0) mof[b1] = m;
     }
     auto live_row = [&](int b1, int s1p) { return mof[b1] < 0 ? int64_t(-1) : tb[(size_t)b1 * nm + mof[b1]].row[s1p]; };
+    // RightPart blocks by output state, in the order of (b1, sigma2)
+    struct Read {
+      int b1, s2;
+      int64_t ro;
+    };
+    std::vector<std::vector<Read>> reads(d);
+    for (int b1 = 0; b1 < D; ++b1) {
+      if (mof[b1] < 0) continue;
+      for (int s2 = 0; s2 < d; ++s2) {
+        const int t = csec[(size_t)mof[b1] * d + s2];
+        if (t < 0) continue;
+        for (int s2p = 0; s2p < d; ++s2p) {
+          const int64_t ro = rp_at(b1, s2, s2p, t);
+          if (ro >= 0) reads[s2p].push_back(Read{b1, s2, ro});
+        }
+      }
+    }
     for (size_t i = 0; i < by_off.size();) {
       const int first = by_off[i];
       if (th.rowoff[mp][first] < 0) {
@@ -1001,25 +1018,20 @@ int Heff::build_plans() {
         task.n = (int32_t)A2.sdim[tp];
         task.ldc = (int32_t)th.ncols[mp];
         task.t0 = (int32_t)stage2.terms.size();
-        for (int b1 = 0; b1 < D; ++b1) {
-          const int64_t row = live_row(b1, first);
+        for (const Read& q : reads[s2p]) {
+          const int64_t row = live_row(q.b1, first);
           if (row < 0) continue;
-          const int m = mof[b1];
-          const TBlock& B = tb[(size_t)b1 * nm + m];
-          for (int s2 = 0; s2 < d; ++s2) {
-            const int t = csec[(size_t)m * d + s2];
-            const int64_t ro = t < 0 ? -1 : rp_at(b1, s2, s2p, t);
-            if (ro < 0) continue;
-            GemmTerm tm{};
-            tm.a_off = t_base[(size_t)b1 * nm + m] + row * B.cols + B.col[s2];
-            tm.lda = (int32_t)B.cols;
-            tm.k = (int32_t)A2.sdim[t];
-            tm.b_off = ro;
-            tm.ldb = (int32_t)A2.sdim[tp];
-            stage2.terms.push_back(tm);
-            flops_executed += 8.0 * task.m * (double)task.n * tm.k;
-            fl[mp] += 8.0 * task.m * (double)task.n * tm.k;
-          }
+          const int m = mof[q.b1];
+          const TBlock& B = tb[(size_t)q.b1 * nm + m];
+          GemmTerm tm{};
+          tm.a_off = t_base[(size_t)q.b1 * nm + m] + row * B.cols + B.col[q.s2];
+          tm.lda = (int32_t)B.cols;
+          tm.k = (int32_t)A2.sdim[csec[(size_t)m * d + q.s2]];
+          tm.b_off = q.ro;
+          tm.ldb = (int32_t)A2.sdim[tp];
+          stage2.terms.push_back(tm);
+          flops_executed += 8.0 * task.m * (double)task.n * tm.k;
+          fl[mp] += 8.0 * task.m * (double)task.n * tm.k;
         }
         task.t1 = (int32_t)stage2.terms.size();
         stage2.tasks.push_back(task);  // a task without terms writes zeros

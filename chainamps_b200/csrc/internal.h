@@ -193,8 +193,9 @@ struct GemmTiles {
 struct GemmPlan {
   std::vector<GemmTask> tasks;
   std::vector<GemmTerm> terms;
-  GemmTask* d_tasks = nullptr;
+  GemmTask* d_tasks = nullptr;  // the allocation of upload: tasks, terms and the first t64 tiles
   GemmTerm* d_terms = nullptr;
+  GemmTile* d_tiles0 = nullptr;
   double flops = 0.0;
   bool nsplit = false;  // tasks use the two-level N index (n_in > 0)
   bool a_real = false;  // the A operand's imaginary plane is zero

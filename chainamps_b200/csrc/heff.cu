@@ -1369,10 +1369,14 @@ static void tridiag_lowest(int k, const double* a, const double* b, double* lam,
   y = z;
 }
 
-// Vectors up to this length run one Lanczos step ahead of the host.  The step
-// that a cycle's end wastes costs as much as the host's turns of about 15
-// steps at 1M entries (matvec and passes 0.5 to 0.8 ms, a turn 40 to 60 us).
-constexpr int64_t kStepAhead = int64_t(1) << 20;
+// Steps that take less than this on the device are issued one ahead of the
+// host.  That hides the host's turn, 5 us of a step with the split operator and
+// 25 us of an FP64 one, but a cycle's end wastes a step.
+// Eigensolve of a growth step with never, short and all steps ahead, ms: XXZ
+// chain at chi = 100, mixed, 2.76, 2.45, 2.46; ladder, mixed, chi = 64 7.20, 6.92,
+// 6.93, chi = 125 16.18, 16.04, 16.23, chi = 165 24.19, 24.21, 24.38; Ising chains,
+// chi = 6, mixed (1.4 ms a step) 137.8, 138.0, 140.4.
+constexpr float kStepAheadMs = 0.2f;
 
 // Restarted Lanczos with full re-orthogonalisation (the local three-term
 // step, then one classical Gram-Schmidt pass against the whole basis),
@@ -1458,6 +1462,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
   double lam = 0.0;
   bool converged = false;
   std::vector<double> al, be, ycoef;
+  float step_ms[2] = {HUGE_VALF, HUGE_VALF};  // the last step's device time, FP64 and split
   for (int cycle = 0; cycle < max_cycles && !converged; ++cycle) {
     ++eig_stats.cycles;
     CMPS_CUDA(cudaMemcpyAsync(vre(0), x.d, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));
@@ -1498,16 +1503,17 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
     };
     int issued = 0;
     for (int j = 0; j < kdim; ++j) {
-      // Short vectors: the next step is issued before this one's coefficients
-      // are read (it needs them on the device only), so that the GPU does not
-      // wait for the host's turn, 40 us or so.  A cycle that ends at this step
+      const int kind = all_fp64 || j == 0 ? 0 : 1;
+      // Short steps: the next one is issued before this one's coefficients are
+      // read (it needs them on the device only).  A cycle that ends at this step
       // drops the extra one: its vector lies past the basis.
-      const int upto = n <= kStepAhead && (all_fp64 || j > 0) ? std::min(j + 1, kdim - 1) : j;
+      const int upto = (all_fp64 || j > 0) && step_ms[kind] < kStepAheadMs ? std::min(j + 1, kdim - 1) : j;
       while (issued <= upto) CMPS_TRY(issue(issued++));
       cudaEvent_t* e = ev + 3 * (j & 1);
       CMPS_CUDA(cudaEventSynchronize(e[2]));
       ++nmv;
       CMPS_TRY(count_matvec(j));
+      CMPS_CUDA(cudaEventElapsedTime(&step_ms[kind], e[0], e[2]));
       const double a = h_ab[2 * (j & 1)], b = h_ab[2 * (j & 1) + 1];
       al.push_back(a);
       be.push_back(b);

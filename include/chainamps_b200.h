@@ -262,8 +262,8 @@ int cmps_heff_eigs(cmps_heff* h, const double* guess, double tol, int max_restar
 /* Work of the last cmps_heff_eigs call on this handle (no reference
  * counterpart; diagnostics).  With CMPS_SPLIT_TF32 each restart cycle opens
  * with one FP64 matvec and continues with split-TF32 ones; with CMPS_FP64
- * every matvec is FP64.  The counts hold every matvec that ran: for short
- * vectors the solver issues a step ahead of its convergence test, so up to one
+ * every matvec is FP64.  The counts hold every matvec that ran: where steps are
+ * short the solver issues a step ahead of its convergence test, so up to one
  * per cycle more than cmps_heff_eigs reports as applications.  ms3 = device time
  * of {split matvecs, FP64 matvecs, whole solve} (CUDA events).  Any output pointer may be NULL. */
 int cmps_heff_eigs_stats(const cmps_heff* h, int* split_matvecs, int* fp64_matvecs, int* cycles, double* ms3);

@@ -813,13 +813,13 @@ int build_canonical_tc(Heff& H) {
     // Tiles of a group of tasks that read the same A rows go row tile by row
     // tile across the group, so the tiles that run at the same time (dealt
     // round-robin to the SMs) share their A tiles in L2.  Where the
-    // number of tasks divides 148 (4 in stage R of the Ising chains) an SM would
+    // number of tasks divides that of the SMs (4 in stage R of the Ising chains) an SM would
     // get the same task, heavy or light, in every row tile: the tasks' order
     // then rotates from row tile to row tile.
     for (auto& g : groups) {
       int32_t mmax = 0;
       for (int32_t t : g.second) mmax = std::max(mmax, p.tasks[t].m);
-      const size_t shift = 148 % g.second.size() == 0 ? 1 : 0;
+      const size_t shift = tc::num_sms() % g.second.size() == 0 ? 1 : 0;
       size_t turn = 0;
       for (int32_t m0 = 0; m0 < mmax; m0 += 128, turn += shift)
         for (size_t i = 0; i < g.second.size(); ++i) {

@@ -373,14 +373,15 @@ int Heff::allowed_indices(int64_t* host_out) const {
   return rc;
 }
 
-// ARPACK order -> sector blocks: CTA = (group of <= 32 columns, 32 rows).
+// ARPACK order <-> sector blocks: CTA = (group of <= 32 columns, 64 rows in the
+// gather, 32 in the scatter).
 // Reads run down each ARPACK column (contiguous), writes along theta rows
 // (the group's columns are consecutive theta columns).
 // HBM bound (16 bytes in, 16 out per entry).  Two dependent reads of
-// descriptors stand before the data (four before: gather 0.27 ms at 33.5M
-// entries, now 0.205).  The gather takes the tile's 64 rows in one CTA, so that
-// more reads are in flight; the scatter gives each half of them a CTA of its own
-// (64 rows there: 0.30 against 0.257 ms).
+// descriptors stand before the data: gather 0.207 ms and scatter 0.190 ms at
+// 33.5M entries, 0.27 and 0.26 with four.  The gather takes the tile's 64 rows in
+// one CTA, so that more reads are in flight; the scatter, which reads short runs,
+// gives each half of them a CTA of its own.
 template <bool PACK>
 __global__ void __launch_bounds__(256) k_pack_tiles(const Heff::PackTile* __restrict__ tiles,
                                                     const Heff::PackGroup* __restrict__ groups,
@@ -1441,7 +1442,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
   if (have_start) CMPS_TRY(ops.norm2(x.re(), x.im(), &nrm0, st));
   if (!have_start || !(nrm0 > 1e-300)) CMPS_TRY(ops.random(x.re(), x.im(), 0x5eed1234ULL, st));
   CMPS_TRY(ops.mdot_dev(nullptr, nullptr, 0, 0, x.re(), x.im(), nrm, st));
-  CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, true, x.re(), x.im(), st));
+  CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, x.re(), x.im(), st));
   h_ab[4] = 1.0;  // a cycle's first basis vector is normalised
   CMPS_CUDA(cudaMemcpyAsync(ops.lanczos_coef().scale, h_ab + 4, sizeof(double), cudaMemcpyHostToDevice, st));
 
@@ -1558,7 +1559,7 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
       ycoef[j] *= be[j - 1] > 1e-14 * std::max(1.0, std::fabs(al[j - 1])) ? 1.0 / be[j - 1] : 0.0;
     CMPS_TRY(ops.combine(kv.d, kv.d + n, ldv, k, ycoef.data(), x.re(), x.im(), st));
     CMPS_TRY(ops.mdot_dev(nullptr, nullptr, 0, 0, x.re(), x.im(), nrm, st));
-    CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, true, x.re(), x.im(), st));
+    CMPS_TRY(ops.scale_dev(x.re(), x.im(), nrm, x.re(), x.im(), st));
     if (issued > k) {  // a step issued ahead and dropped: its matvec has run all the same
       CMPS_CUDA(cudaEventSynchronize(ev[3 * (k & 1) + 1]));
       CMPS_TRY(count_matvec(k));

@@ -64,11 +64,14 @@ inline cudaError_t dmalloc(T** p, size_t bytes) {
 // SVD's worker threads launch the same kernels concurrently.
 int ensure_smem_optin(const void* func, int bytes);
 
-// Launches of the matvec and the Lanczos passes: programmatic dependent launch,
-// so that a kernel's CTAs are set up while the one before it drains.  Such a
-// kernel calls grid_wait() before it touches memory that another kernel reads or
-// writes (descriptors of a plan may be read before).  On the XXZ chain at chi =
-// 100 a matvec of four such launches takes 22.7 us instead of 31.8.
+// Launches of the matvec and the Lanczos passes: programmatic dependent launch.
+// No kernel triggers its dependents itself, so the next one starts when all CTAs
+// of the one before it have ended: what is gained is its launch and the wait for
+// the other's last writes, while it reads its plan.  Such a kernel calls
+// grid_wait() before it touches memory that another kernel reads or writes
+// (descriptors of a plan, whose upload was waited for, may be read before).  On
+// the XXZ chain at chi = 100 a matvec of four such launches takes 22 us instead
+// of 32.
 template <class... P, class... A>
 inline cudaError_t launch_chained(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, cudaStream_t st,
                                   A&&... args) {

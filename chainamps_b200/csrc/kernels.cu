@@ -1,6 +1,6 @@
 // Memory-bound kernels of the hot path: block AXPY lists (LeftPart /
 // RightPart formation) and the FP64 vector kernels of the device Krylov
-// solver.  All are grid-stride loops sized to a multiple of the SM count.
+// solver.  These are grid-stride loops over a few CTAs per SM.
 #include <cuda_runtime.h>
 #include <stdint.h>
 
@@ -95,34 +95,6 @@ __global__ void k_reduce_rows(const double* __restrict__ partial, int nb, int ro
     __syncthreads();
   }
   if (threadIdx.x == 0) out[r] = red[0];
-}
-
-// w -= sum_j h_j V_j  (h complex, k <= 64 in constant-like global memory)
-__global__ void k_multiaxpy(const double* __restrict__ Vr, const double* __restrict__ Vi, int64_t ldv, int k,
-                            const double* __restrict__ h, double* __restrict__ wr, double* __restrict__ wi,
-                            int64_t n, double sign) {
-  __shared__ double hs[2 * 128];
-  for (int j = threadIdx.x; j < 2 * k; j += blockDim.x) hs[j] = h[j];
-  __syncthreads();
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    double xr = 0.0, xi = 0.0;
-    for (int j = 0; j < k; ++j) {
-      double hr = hs[2 * j], hi = hs[2 * j + 1];
-      double vr = Vr[(int64_t)j * ldv + i], vi = Vi[(int64_t)j * ldv + i];
-      xr += hr * vr - hi * vi;
-      xi += hr * vi + hi * vr;
-    }
-    wr[i] += sign * xr;
-    wi[i] += sign * xi;
-  }
-}
-
-__global__ void k_scale_copy(const double* __restrict__ xr, const double* __restrict__ xi, double s,
-                             double* __restrict__ yr, double* __restrict__ yi, int64_t n) {
-  for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
-    yr[i] = s * xr[i];
-    yi[i] = s * xi[i];
-  }
 }
 
 __device__ __forceinline__ uint64_t mix64(uint64_t x) {
@@ -582,13 +554,12 @@ k_lanczos_update(const double* __restrict__ U, int64_t ldv, const double* __rest
   }
 }
 
-// y = s * x with s read from the device; `inv_sqrt` takes s = 1 / sqrt(*p)
-// (0 when *p is not positive).
+// y = x / sqrt(*p), 0 when *p is not positive.
 __global__ void k_scale_dev(const double* __restrict__ xr, const double* __restrict__ xi,
-                            const double* __restrict__ p, int inv_sqrt, double* __restrict__ yr,
-                            double* __restrict__ yi, int64_t n) {
+                            const double* __restrict__ p, double* __restrict__ yr, double* __restrict__ yi,
+                            int64_t n) {
   const double v = *p;
-  const double s = inv_sqrt ? (v > 0.0 ? 1.0 / sqrt(v) : 0.0) : v;
+  const double s = v > 0.0 ? 1.0 / sqrt(v) : 0.0;
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x) {
     yr[i] = s * xr[i];
     yi[i] = s * xi[i];
@@ -643,25 +614,10 @@ int VecOps::multidot(const double* Vr, const double* Vi, int64_t ldv, int k, con
   return CMPS_OK;
 }
 
-int VecOps::multiaxpy(const double* Vr, const double* Vi, int64_t ldv, int k, const double* h_host, double* wr,
-                      double* wi, double sign, cudaStream_t st) {
-  if (k > 128) return fail(CMPS_ERR_ARG, "krylov dimension above 128");
-  CMPS_CUDA(cudaMemcpyAsync(d_small + 256, h_host, sizeof(double) * 2 * k, cudaMemcpyHostToDevice, st));
-  k_multiaxpy<<<grid_for(n, 256), 256, 0, st>>>(Vr, Vi, ldv, k, d_small + 256, wr, wi, n, sign);
-  CMPS_CUDA(cudaGetLastError());
-  return CMPS_OK;
-}
-
 int VecOps::norm2(const double* xr, const double* xi, double* out, cudaStream_t st) {
   double h[2];
   CMPS_TRY(multidot(xr, xi, 0, 1, xr, xi, h, st));
   *out = h[0];
-  return CMPS_OK;
-}
-
-int VecOps::scale_copy(const double* xr, const double* xi, double s, double* yr, double* yi, cudaStream_t st) {
-  k_scale_copy<<<grid_for(n, 256), 256, 0, st>>>(xr, xi, s, yr, yi, n);
-  CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }
 
@@ -772,9 +728,8 @@ int VecOps::lanczos(const double* U, int64_t ldv, const double* yr, const double
   return lanczos_step<false, 1>(*this, U, ldv, yr, yi, unit, j, outr, outi, host, st);
 }
 
-int VecOps::scale_dev(const double* xr, const double* xi, const double* d_s, bool inv_sqrt, double* yr, double* yi,
-                      cudaStream_t st) {
-  k_scale_dev<<<grid_for(n, 256), 256, 0, st>>>(xr, xi, d_s, inv_sqrt ? 1 : 0, yr, yi, n);
+int VecOps::scale_dev(const double* xr, const double* xi, const double* d_sq, double* yr, double* yi, cudaStream_t st) {
+  k_scale_dev<<<grid_for(n, 256), 256, 0, st>>>(xr, xi, d_sq, yr, yi, n);
   CMPS_CUDA(cudaGetLastError());
   return CMPS_OK;
 }

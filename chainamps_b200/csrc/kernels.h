@@ -13,9 +13,9 @@ struct LanczosCoef {
   double *a, *h, *beta, *scale, *nrm2;
 };
 
-// Planar FP64 complex vectors of a fixed length n; reductions are two-pass
-// (per-CTA partials, then a fixed-order reduction) so results are
-// deterministic run to run.
+// Planar FP64 complex vectors of a fixed length n.  Reductions add one partial
+// sum per CTA in a fixed order, in a second launch or in the CTA that finishes
+// last, so results are deterministic run to run.
 struct VecOps {
   int64_t n = 0;
   int nb = 0;
@@ -27,11 +27,7 @@ struct VecOps {
   // h[j] = <V_j, w> (conjugate-linear in V), k vectors with stride ldv; h_host gets 2k doubles.
   int multidot(const double* Vr, const double* Vi, int64_t ldv, int k, const double* wr, const double* wi,
                double* h_host, cudaStream_t st);
-  // w += sign * sum_j h_j V_j
-  int multiaxpy(const double* Vr, const double* Vi, int64_t ldv, int k, const double* h_host, double* wr,
-                double* wi, double sign, cudaStream_t st);
   int norm2(const double* xr, const double* xi, double* out, cudaStream_t st);
-  int scale_copy(const double* xr, const double* xi, double s, double* yr, double* yi, cudaStream_t st);
   int random(double* re, double* im, uint64_t seed, cudaStream_t st);
   // y = sum_j c_j V_j, c real
   int combine(const double* Vr, const double* Vi, int64_t ldv, int k, const double* c_host, double* yr,
@@ -49,16 +45,15 @@ struct VecOps {
                      double* wi, double* d_nrm2, cudaStream_t st);
   // Step j of a Lanczos cycle with full re-orthogonalisation (kernels.cu):
   // basis vectors U_0 .. U_j at U + i ldv (real plane, imaginary plane n
-  // further), y = H U_j, or H V_j where `unit` is set; the next vector into (outr, outi) unless they are null,
-  // alpha_j and beta_j into host[0..1] (pinned memory) once the stream has come
-  // this far.  The cycle's first scale, lanczos_coef().scale[0], is the caller's.
+  // further), y = H U_j, or H V_j where `unit` is set; the next vector into
+  // (outr, outi) unless they are null, alpha_j and beta_j into host[0..1] (pinned
+  // memory) once the stream has come this far.  The cycle's first scale, lanczos_coef().scale[0], is the caller's.
   int lanczos(const double* U, int64_t ldv, const double* yr, const double* yi, bool unit, int j, double* outr,
               double* outi, double* host, cudaStream_t st);
   LanczosCoef lanczos_coef() const;
   unsigned* d_count = nullptr;  // CTAs of the current launch that have finished
-  // y = s x with s = *d_s, or s = 1 / sqrt(*d_s) when inv_sqrt.
-  int scale_dev(const double* xr, const double* xi, const double* d_s, bool inv_sqrt, double* yr, double* yi,
-                cudaStream_t st);
+  // y = x / sqrt(*d_sq)
+  int scale_dev(const double* xr, const double* xi, const double* d_sq, double* yr, double* yi, cudaStream_t st);
   int phase_drop(double* re, double* im, double pr, double pi, double thr, cudaStream_t st);
 };
 

@@ -1463,7 +1463,9 @@ int Heff::eigs(const double* guess, double tol, int max_restarts, int kdim, doub
   double lam = 0.0;
   bool converged = false;
   std::vector<double> al, be, ycoef;
-  float step_ms[2] = {HUGE_VALF, HUGE_VALF};  // the last step's device time, FP64 and split
+  // the last step's device time, FP64 and split; before the first one, short
+  // for vectors whose passes are
+  float step_ms[2] = {n <= 32768 ? 0.f : HUGE_VALF, HUGE_VALF};
   for (int cycle = 0; cycle < max_cycles && !converged; ++cycle) {
     ++eig_stats.cycles;
     CMPS_CUDA(cudaMemcpyAsync(vre(0), x.d, sizeof(double) * 2 * n, cudaMemcpyDeviceToDevice, st));

@@ -824,7 +824,8 @@ int launch(int mode, const TcPlan& p, float* out32, int64_t out32_plane, double*
   const int ntiles = (int)p.tiles.size();
   const unsigned grid = (unsigned)std::min(ntiles, num_sms());
   if (mode == 1 || mode == 3 || mode == 4) {
-    if (!p.d_amaps) return fail(CMPS_ERR_STATE, "tcgen05: no A tensor maps");
+    // a plan whose tasks have no terms at all writes zeros and reads no operand
+    if (!p.d_amaps && !p.terms.empty()) return fail(CMPS_ERR_STATE, "tcgen05: no A tensor maps");
     auto kern = mode == 1 ? tc_split_gemm<1> : mode == 3 ? tc_split_gemm<3> : tc_split_gemm<4>;
     const int smem = mode == 3 ? smem_bytes_of<3>() : kSmemBytes;
     CMPS_TRY(ensure_smem_optin((const void*)kern, smem));
@@ -832,7 +833,7 @@ int launch(int mode, const TcPlan& p, float* out32, int64_t out32_plane, double*
     CMPS_CUDA(launch_chained(kern, dim3(grid), dim3(threads), (size_t)smem, st, p.d_tiles, ntiles, p.d_tasks, p.d_terms,
                              p.d_amaps, p.d_bmaps, nullptr, nullptr, 0, out32, out32_plane, out64, out64_plane, d_err));
   } else if (mode == 2) {
-    if (!ain || !p.d_adescs) return fail(CMPS_ERR_STATE, "tcgen05 mode 2: no A operand");
+    if ((!ain || !p.d_adescs) && !p.terms.empty()) return fail(CMPS_ERR_STATE, "tcgen05 mode 2: no A operand");
     CMPS_TRY(ensure_smem_optin((const void*)tc_split_gemm<2>, kSmemBytes));
     CMPS_CUDA(launch_chained(tc_split_gemm<2>, dim3(grid), dim3(threads_of<2>()), (size_t)kSmemBytes, st, p.d_tiles,
                              ntiles, p.d_tasks, p.d_terms, nullptr, p.d_bmaps, p.d_adescs, ain, a_plane, out32,

@@ -153,3 +153,74 @@ def test_infinite_component():
     assert got[0].real == np.inf
     del h
     ctx.close()
+
+
+PRECISIONS = ["CMPS_FP64", "CMPS_SPLIT_TF32", "CMPS_SPLIT_BF16"]
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_zero_operator(precision):
+    """One MPO entry, into a slot that no entry leaves: H = 0, and no element of T
+    is both produced and read."""
+    import chainamps_b200 as ca
+    from chainamps_b200 import models
+    rng, rules = np.random.default_rng(4), (0,)
+    bl, br, bq = _bond([5, 9]), _bond([8, 3]), np.zeros((2, 1), np.int64)
+    W = np.zeros((1, 2, 1, 2), np.complex128)
+    W[0, 0, 0, 1] = 1.0
+    L = models.random_environment(rng, rules, bl, bq, [0, 1], right=False)
+    R = models.random_environment(rng, rules, br, bq, [0, 1], right=True)
+    ctx = ca.Context(0)
+    h = ca.TwoVertexComponents(ctx, rules, L, models.mpo_tensor(np.zeros((1, 1), np.int64), W, bq), R)
+    h.set_order(ca.CMPS_ORDER_FOLDED)
+    h.set_precision(getattr(ca, precision))
+    x = rng.standard_normal(h.n) + 1j * rng.standard_normal(h.n)
+    assert np.array_equal(h.multiply(x), np.zeros(h.n))
+    del h
+    ctx.close()
+
+
+@pytest.mark.parametrize("precision", PRECISIONS)
+def test_owned_sector_that_nothing_reaches(precision):
+    """States of charge 0 and 1, the MPO acts on charge 0 only.  In the sector of
+    middle charge 0 the left vertex can carry charge 0 but the right one
+    cannot: its rows of T are produced, none of its columns are read.  Owned
+    alone, each sector is what it is in the whole matvec."""
+    import torch
+    import chainamps_b200 as ca
+    from chainamps_b200 import models
+    rng, rules = np.random.default_rng(5), (0,)
+    ch, bq = np.array([[0], [1]], np.int64), np.zeros((1, 1), np.int64)
+    W = np.zeros((2, 1, 2, 1), np.complex128)
+    W[0, 0, 0, 0] = 1.0
+    bl, br = _bond([4, 6]), _bond([7, 5]) + 1
+    L = models.random_environment(rng, rules, bl, bq, [0], right=False)
+    R = models.random_environment(rng, rules, br, bq, [0], right=True)
+    ctx = ca.Context(0)
+    h = ca.TwoVertexComponents(ctx, rules, L, models.mpo_tensor(ch, W, bq), R)
+    h.set_order(ca.CMPS_ORDER_FOLDED)
+    h.set_precision(getattr(ca, precision))
+    x = torch.randn(h.n, dtype=torch.complex128, device="cuda", generator=torch.Generator("cuda").manual_seed(1))
+    vin, vout = (torch.zeros(2 * h.n, dtype=torch.float64, device="cuda") for _ in range(2))
+    torch.cuda.synchronize()
+    h.theta_from_arpack_device(x.data_ptr(), vin.data_ptr(), 0)
+    h.multiply_theta_device(vin.data_ptr(), vout.data_ptr(), 0)
+    torch.cuda.synchronize()
+    whole = vout.cpu().numpy().copy()
+    base, _ = h.sector_table()
+    seen = set()
+    for m in range(len(base) - 1):
+        own = np.zeros(len(base) - 1, np.uint8)
+        own[m] = 1
+        h.set_owned(own)
+        vout.fill_(7.0)
+        torch.cuda.synchronize()
+        h.multiply_theta_device(vin.data_ptr(), vout.data_ptr(), 0)
+        torch.cuda.synchronize()
+        got, part = vout.cpu().numpy(), slice(base[m], base[m + 1])
+        for plane in (0, h.n):
+            assert np.array_equal(got[plane:][part], whole[plane:][part])
+        seen.add(bool(np.any(whole[part])))
+    assert seen == {True, False}
+    del h
+    ctx.close()
